@@ -397,6 +397,9 @@ decode_attention_kernel(const bf16* qkv, const W* __restrict__ q_weight,
             cp_async_16(values_to + at, v_base + offset, slot >= 0);
         }
     };
+    // Keys of earlier steps are there before the kernel ahead of this one ends; with cached_new the
+    // last ones are that kernel's own (a short prompt portion, its keys stored a launch ago).
+    if (cached_new) pdl_wait();
 #pragma unroll
     for (int i = 0; i < DEC_STAGES - 1; ++i) {  // in flight before anything of this step is needed
         if (i < mine) issue(i);
