@@ -1851,7 +1851,7 @@ def attention_tiles_singles(q: torch.Tensor, key_cache: torch.Tensor, value_cach
 # ----------------------------------------------------------------------- GEMM
 def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
                  out_dtype: torch.dtype | None = None) -> torch.Tensor:
-    """a [m, k] . w [n, k]^T on the float32 cores, ascending k."""
+    """a [m, k] . w [n, k]^T on the float32 cores; the order of a sum over k depends on k alone."""
     _need_cuda(a, w)
     if a.dim() != 2 or w.dim() != 2 or a.shape[1] != w.shape[1] or a.dtype != w.dtype:
         raise KernelError("gemm_nt_simt wants a [m, k] and w [n, k] of one dtype")
@@ -1863,9 +1863,15 @@ def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = No
         out = torch.empty((m, n), dtype=out_dtype or a.dtype, device=a.device)
     fn = _fn("gemm_simt", "tvb_gemm_nt_simt",
              [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int,
-              c_int, c_int, c_void_p])
+              c_int, c_int, c_void_p, c_void_p])
+    scratch = None
+    if a.dtype == torch.float32:
+        floats = _fn("gemm_simt", "tvb_gemm_f32_scratch_floats", [c_int, c_int, c_int], c_longlong)(m, n, k)
+        if floats > 0:           # partial sums of the pieces that k is cut into
+            scratch = torch.empty(floats, dtype=torch.float32, device=a.device)
     _check(fn(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0),
-              m, n, k, dtype_tag(a.dtype), dtype_tag(out.dtype), _stream()), "gemm_nt_simt")
+              m, n, k, dtype_tag(a.dtype), dtype_tag(out.dtype), None if scratch is None else scratch.data_ptr(),
+              _stream()), "gemm_nt_simt", 1 if scratch is None else 2)
     return out
 
 
