@@ -351,6 +351,8 @@ __global__ void merge_attention_rows_kernel(const float* __restrict__ scratch, i
                         head_dim, lane);
 }
 
+#include "attention_rows_f32.cuh"
+
 extern "C" int tvb_attention_chunk_keys() { return ATTN_CHUNK; }
 
 // scratch floats the split mode needs: tokens * num_q * max_chunks * (head_dim + 2)
@@ -418,6 +420,22 @@ extern "C" int tvb_attention_rows_masked(const void* q, long long q_token_stride
     RowExtras extras{slopes, sinks, gate_per_head, value_stride > 0 ? value_stride : value_dim,
                      bias_table, bias_rows, segment, softcap};
     const bool wide = head_dim > 32 * ATTN_MAX_DIMS || value_dim > 32 * ATTN_MAX_DIMS;
+    // Plain float32 heads of 64 and 128 in groups of a power of two: the kernels that read a block of keys at a time.
+    const int group = num_q / num_kv;
+    if (dtype == TVB_F32 && head_dim == value_dim && (head_dim == 64 || head_dim == 128) && extras.value_stride == value_dim &&
+        !gate && !slopes && !sinks && !bias_table && segment == 0 && softcap == 0.0f && (keep_first == 0 || window == 0) &&
+        (group == 1 || group == 2 || group == 4 || group == 8) &&
+        ((reinterpret_cast<uintptr_t>(key_cache) | reinterpret_cast<uintptr_t>(value_cache)) & 15) == 0) {
+        const F32Args args{(const float*)q, q_token_stride, (const float*)key_cache, (const float*)value_cache, block_tables,
+                           table_stride, token_row, positions, (float*)out, out_token_stride, scratch, max_chunks, tokens,
+                           num_q, num_kv, page_size, window, scale};
+        const int status = launch_f32_of(head_dim, group, args, s);
+        if (status != 0 || max_chunks == 0) return status;
+        merge_attention_rows_kernel<float, ATTN_MAX_DIMS><<<(unsigned)blocks, ATTN_WARPS * 32, 0, s>>>(
+            scratch, max_chunks, token_row, positions, (float*)out, out_token_stride, nullptr, 0, tokens, num_q, value_dim,
+            window, 0, extras);
+        return tvb_last_error();
+    }
 #define LAUNCH_ROWS(T, DIMS)                                                                             \
     launch_rows<T, DIMS>(q, q_token_stride, key_cache, value_cache, block_tables, table_stride, token_row, \
                          positions, out, out_token_stride, gate, gate_token_stride, scratch, max_chunks,   \
