@@ -15,8 +15,16 @@
 // u = ((word >> 9) + 0.5) / 2^23, noise = -log(u).  A request's tokens thus do not
 // depend on what else is in the batch or on the order of the rows.
 //
-// No sort: thresholds are found by bisection over the ordered bit pattern of the
-// scores, each probe being one pass over the row.
+// No sort: the thresholds are found three bits of the ordered bit pattern at a time.  A pass counts (top-k) or adds
+// up (top-p) the tokens of the eight continuations of the bits found so far; eleven passes settle all 32 bits, and
+// the last one also says how many tokens equal the threshold.  A CTA keeps its part of the row's scores in shared
+// memory, each thread its own four tokens of every 2,048, so a pass reads nothing from global memory and costs two block barriers and
+// one of the cluster.  Rows too long for that (more than about 430,000 tokens) read the logits in every pass.
+//
+// Bound by the passes' barriers and compares.  Measured over 151,936 tokens (us; one bit a pass over the logits in L2 /
+// this): 48 rows, half of them greedy, a quarter top-k 50, a quarter top-p 0.95 684 / 140; one row of top-k 50 499 / 53,
+// of top-p 0.95 647 / 77, of both 1,016 / 90; 64 rows of both 1,096 / 325; one greedy row 4.9 / 5.0, 64 greedy rows
+// 11.6 / 17.6 (the shared memory that they do not use leaves two CTAs an SM).
 #include "common.cuh"
 
 #include <cstdint>
@@ -24,9 +32,12 @@
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
 
-#define SAMPLE_THREADS 256
+#define SAMPLE_THREADS 512
 #define SAMPLE_WARPS (SAMPLE_THREADS / 32)
 #define SAMPLE_CTAS 8           // CTAs (one cluster) that share a row
+#define SAMPLE_DIGIT 3          // bits of the threshold that a pass settles
+#define SAMPLE_BINS (1 << SAMPLE_DIGIT)
+#define SAMPLE_STAGED_BYTES (208 * 1024)
 
 __device__ __forceinline__ uint32_t ordered_key(float f) {
     const uint32_t b = __float_as_uint(f);
@@ -51,10 +62,12 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t
 // memory, and one cluster barrier; the buffers alternate, so a slot is not written again before
 // every CTA has read it (it has to pass the barrier in between).
 struct SampleShared {
-    float warp_f[SAMPLE_WARPS];
+    uint32_t warp_key[SAMPLE_WARPS];
     int warp_i[SAMPLE_WARPS];
-    float part_f[2][SAMPLE_CTAS];
+    uint32_t part_key[2][SAMPLE_CTAS];
     int part_i[2][SAMPLE_CTAS];
+    uint32_t warp_bins[SAMPLE_BINS][SAMPLE_WARPS];
+    uint32_t part_bins[2][SAMPLE_CTAS][SAMPLE_BINS];       // counts, or sums as their bits
 };
 
 struct RowTeam {
@@ -63,91 +76,102 @@ struct RowTeam {
     int rank;
     int phase;
 
-    // partial (f, i) of this CTA, held by thread 0, to every CTA of the cluster; then the barrier
-    __device__ __forceinline__ void publish(float f, int i) {
-        if (threadIdx.x == 0) {
-#pragma unroll
-            for (int r = 0; r < SAMPLE_CTAS; ++r) {
-                SampleShared* other = cluster.map_shared_rank(sh, r);
-                other->part_f[phase][rank] = f;
-                other->part_i[phase][rank] = i;
-            }
-        }
-        cluster.sync();
-    }
-
-    __device__ __forceinline__ int sum(int v) {
+    // count of this CTA alone
+    __device__ __forceinline__ int local_sum(int v) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-        for (int delta = 16; delta > 0; delta >>= 1) v += __shfl_xor_sync(0xffffffffu, v, delta);
+        v = __reduce_add_sync(0xffffffffu, v);
         __syncthreads();
         if (lane == 0) sh->warp_i[warp] = v;
         __syncthreads();
         int total = 0;
 #pragma unroll
         for (int w = 0; w < SAMPLE_WARPS; ++w) total += sh->warp_i[w];
-        publish(0.0f, total);
-        total = 0;
-#pragma unroll
-        for (int r = 0; r < SAMPLE_CTAS; ++r) total += sh->part_i[phase][r];
-        phase ^= 1;
         return total;
     }
 
-    // warps, then CTAs, in a fixed order
-    __device__ __forceinline__ float sum(float v) {
+    // The eight bins of every thread, added up: lanes, warps, then CTAs, in a fixed order.  part_bins[the phase returned]
+    // holds every CTA's sums afterwards; it stays until the next but one call.
+    template <typename V> __device__ __forceinline__ int sum_bins(const V* bins, V* totals) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        v = warp_sum(v);
-        __syncthreads();
-        if (lane == 0) sh->warp_f[warp] = v;
-        __syncthreads();
-        float total = 0.0f;
 #pragma unroll
-        for (int w = 0; w < SAMPLE_WARPS; ++w) total = __fadd_rn(total, sh->warp_f[w]);
-        publish(total, 0);
-        total = 0.0f;
+        for (int b = 0; b < SAMPLE_BINS; ++b) {
+            uint32_t bits;
+            if constexpr (sizeof(V) == 4 && V(0.5f) != V(0)) bits = __float_as_uint(warp_sum(bins[b]));
+            else bits = __reduce_add_sync(0xffffffffu, (uint32_t)bins[b]);
+            if (lane == b) sh->warp_bins[b][warp] = bits;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const int b = lane % SAMPLE_BINS;
+            V total = 0;
 #pragma unroll
-        for (int r = 0; r < SAMPLE_CTAS; ++r) total = __fadd_rn(total, sh->part_f[phase][r]);
+            for (int w = 0; w < SAMPLE_WARPS; ++w) total = add(total, value_of<V>(sh->warp_bins[b][w]));
+            // lanes 8 r .. 8 r + 7 write to the CTAs r and r + 4
+#pragma unroll
+            for (int r = lane / SAMPLE_BINS; r < SAMPLE_CTAS; r += 32 / SAMPLE_BINS)
+                cluster.map_shared_rank(sh, r)->part_bins[phase][rank][b] = bits_of(total);
+        }
+        cluster.sync();
+#pragma unroll
+        for (int b = 0; b < SAMPLE_BINS; ++b) {
+            V total = value_of<V>(sh->part_bins[phase][0][b]);
+#pragma unroll
+            for (int r = 1; r < SAMPLE_CTAS; ++r) total = add(total, value_of<V>(sh->part_bins[phase][r][b]));
+            totals[b] = total;
+        }
+        const int used = phase;
         phase ^= 1;
-        return total;
+        return used;
+    }
+    static __device__ __forceinline__ int add(int a, int b) { return a + b; }
+    static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+    static __device__ __forceinline__ uint32_t bits_of(int v) { return (uint32_t)v; }
+    static __device__ __forceinline__ uint32_t bits_of(float v) { return __float_as_uint(v); }
+    template <typename V> static __device__ __forceinline__ V value_of(uint32_t bits) {
+        if constexpr (V(0.5f) != V(0)) return __uint_as_float(bits); else return (int)bits;
     }
 
-    // argmax of (value, smaller index wins ties); every thread of every CTA gets it
+    // (key, index) of the largest key, the smaller index among equals
+    static __device__ __forceinline__ void warp_best(uint32_t& key, int& index) {
+        const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+        index = (int)__reduce_min_sync(0xffffffffu, key == top ? (uint32_t)index : 0x7fffffffu);
+        key = top;
+    }
+
+    // argmax of (value, smaller index wins ties) of values that are numbers or -inf; every thread of every CTA gets it
     __device__ __forceinline__ void argmax(float& value, int& index) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-        for (int delta = 16; delta > 0; delta >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, value, delta);
-            const int oi = __shfl_xor_sync(0xffffffffu, index, delta);
-            if (ov > value || (ov == value && oi < index)) { value = ov; index = oi; }
-        }
+        uint32_t key = ordered_key(__fadd_rn(value, 0.0f));       // -0 and 0 are equals
+        warp_best(key, index);
         __syncthreads();
-        if (lane == 0) { sh->warp_f[warp] = value; sh->warp_i[warp] = index; }
+        if (lane == 0) { sh->warp_key[warp] = key; sh->warp_i[warp] = index; }
         __syncthreads();
-        value = sh->warp_f[0]; index = sh->warp_i[0];
-#pragma unroll
-        for (int w = 1; w < SAMPLE_WARPS; ++w) {
-            const float ov = sh->warp_f[w];
-            const int oi = sh->warp_i[w];
-            if (ov > value || (ov == value && oi < index)) { value = ov; index = oi; }
+        if (warp == 0) {
+            key = sh->warp_key[lane % SAMPLE_WARPS];
+            index = sh->warp_i[lane % SAMPLE_WARPS];
+            warp_best(key, index);
+            if (lane < SAMPLE_CTAS) {                             // lane r tells CTA r
+                SampleShared* other = cluster.map_shared_rank(sh, lane);
+                other->part_key[phase][rank] = key;
+                other->part_i[phase][rank] = index;
+            }
         }
-        publish(value, index);
-        value = sh->part_f[phase][0]; index = sh->part_i[phase][0];
-#pragma unroll
-        for (int r = 1; r < SAMPLE_CTAS; ++r) {
-            const float ov = sh->part_f[phase][r];
-            const int oi = sh->part_i[phase][r];
-            if (ov > value || (ov == value && oi < index)) { value = ov; index = oi; }
-        }
+        cluster.sync();
+        key = sh->part_key[phase][lane % SAMPLE_CTAS];
+        index = sh->part_i[phase][lane % SAMPLE_CTAS];
+        warp_best(key, index);
+        value = __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key);
         phase ^= 1;
     }
 };
 
-template <typename T>
+// STAGED: the scores stay in shared memory (room for this CTA's part of the row).
+template <typename T, bool STAGED>
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_rows_kernel(const T* logits, int64_t row_stride, int vocab,   // logits: from the kernel before
                    const int* __restrict__ packed, int capacity, int* __restrict__ tokens) {
     __shared__ SampleShared shared;
+    extern __shared__ __align__(16) float staged[];
     RowTeam team{cg::this_cluster(), &shared, (int)(blockIdx.x % SAMPLE_CTAS), 0};
     cluster_arrive();                       // this CTA runs; waited for before the first remote store
     pdl_wait();
@@ -156,37 +180,64 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int vocab,   // logits: 
     // this CTA's part of the row: whole groups of four tokens (they share a block of noise)
     const int part = ((vocab + SAMPLE_CTAS - 1) / SAMPLE_CTAS + 3) / 4 * 4;
     const int begin = min(vocab, team.rank * part), end = min(vocab, begin + part);
+    const int first_quad = begin / 4 + tid, quads_end = (end + 3) / 4;       // begin < end: begin is a multiple of four
+    const bool any = begin < end;
+    const bool wide = sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    // a token that is not there: a bit pattern below every score's (no arithmetic gives it)
+    const float absent = __uint_as_float(0xffffffffu);
 
+    auto load_quad = [&](int quad, float* v) {
+        if (wide && quad * 4 + 4 <= end) {
+            const float4 f = reinterpret_cast<const float4*>(x)[quad];
+            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = quad * 4 + e < end ? to_float<T>(x[quad * 4 + e]) : absent;
+        }
+    };
     float best = -INFINITY;
     int best_index = 0x7fffffff;
-    int scalar_from = begin;
-    if (sizeof(T) == 4 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-        // float32 rows on a 16-byte boundary: four logits a load (begin is a multiple of four)
-        const float4* x4 = reinterpret_cast<const float4*>(x);
-        const int quads_end = end / 4;
-#pragma unroll 4
-        for (int q = begin / 4 + tid; q < quads_end; q += SAMPLE_THREADS) {
-            const float4 v = x4[q];
-            if (v.x > best) { best = v.x; best_index = 4 * q; }
-            if (v.y > best) { best = v.y; best_index = 4 * q + 1; }
-            if (v.z > best) { best = v.z; best_index = 4 * q + 2; }
-            if (v.w > best) { best = v.w; best_index = 4 * q + 3; }
-        }
-        scalar_from = max(begin, quads_end * 4);
-    }
-    for (int i = scalar_from + tid; i < end; i += SAMPLE_THREADS) {
-        const float v = to_float<T>(x[i]);
-        if (v > best || (v == best && i < best_index)) { best = v; best_index = i; }
+    const float temp = __int_as_float(packed[row]);
+    const bool greedy = !(temp > 0.0f);
+#pragma unroll 5
+    for (int quad = first_quad; any && quad < quads_end; quad += SAMPLE_THREADS) {
+        float v[4];
+        load_quad(quad, v);
+        if (STAGED && !greedy) reinterpret_cast<float4*>(staged)[quad - begin / 4] = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (v[e] > best) { best = v[e]; best_index = 4 * quad + e; }     // (absent is greater than nothing)
     }
     cluster_wait();
     team.argmax(best, best_index);
-    const float temp = __int_as_float(packed[row]);
-    if (!(temp > 0.0f) || best_index == 0x7fffffff) {           // the same in every CTA of the row
+    if (greedy || best_index == 0x7fffffff) {           // the same in every CTA of the row
         if (tid == 0 && team.rank == 0) tokens[row] = best_index == 0x7fffffff ? 0 : best_index;
         return;
     }
     const float row_max = best;
-#define SCORE(i) __fdiv_rn(__fsub_rn(to_float<T>(x[i]), row_max), temp)
+    // Four scores of this thread; a token past the row's end comes as `absent`, whose key is 0.
+    auto make_scores = [&](int quad, float* v) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            v[e] = quad * 4 + e < end ? __fdiv_rn(__fsub_rn(v[e], row_max), temp) : absent;
+    };
+    if constexpr (STAGED) {                                      // every thread its own: no barrier
+        for (int quad = first_quad; any && quad < quads_end; quad += SAMPLE_THREADS) {
+            float4& at = reinterpret_cast<float4*>(staged)[quad - begin / 4];
+            float v[4] = {at.x, at.y, at.z, at.w};
+            make_scores(quad, v);
+            at = make_float4(v[0], v[1], v[2], v[3]);
+        }
+    }
+    auto scores_of = [&](int quad, float* v) {
+        if constexpr (STAGED) {
+            const float4 f = reinterpret_cast<const float4*>(staged)[quad - begin / 4];
+            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        } else {
+            load_quad(quad, v);
+            make_scores(quad, v);
+        }
+    };
 
     // ---- top-k: the k-th largest key, then how many of its equals stay
     const int k = packed[2 * capacity + row];
@@ -194,30 +245,64 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int vocab,   // logits: 
     uint32_t k_key = 0;
     int k_index_limit = vocab;
     if (use_k) {
-        for (int bit = 31; bit >= 0; --bit) {
-            const uint32_t candidate = k_key | (1u << bit);
-            int count = 0;
-            for (int i = begin + tid; i < end; i += SAMPLE_THREADS) count += ordered_key(SCORE(i)) >= candidate;
-            if (team.sum(count) >= k) k_key = candidate;
-        }
-        int greater = 0, equal = 0;
-        for (int i = begin + tid; i < end; i += SAMPLE_THREADS) {
-            const uint32_t key = ordered_key(SCORE(i));
-            greater += key > k_key;
-            equal += key == k_key;
-        }
-        greater = team.sum(greater);
-        equal = team.sum(equal);
-        const int wanted = k - greater;
-        if (equal > wanted) {              // ties: the first `wanted` of them by token id
-            int lo = 0, hi = vocab;
-            while (lo < hi) {
-                const int mid = lo + (hi - lo) / 2;
-                int count = 0;
-                for (int i = begin + tid; i < min(end, mid); i += SAMPLE_THREADS) count += ordered_key(SCORE(i)) == k_key;
-                if (team.sum(count) >= wanted) hi = mid; else lo = mid + 1;
+        int above = 0, equal = 0, used = 0;
+        for (int shift = 30; shift >= 0; shift -= SAMPLE_DIGIT) {            // 2 bits, then ten times 3
+            int bins[SAMPLE_BINS], totals[SAMPLE_BINS];
+#pragma unroll
+            for (int b = 0; b < SAMPLE_BINS; ++b) bins[b] = 0;
+            const uint32_t found = shift == 30 ? 0u : k_key >> (shift + SAMPLE_DIGIT);
+            int quad = any ? first_quad : quads_end;
+            while (quad < quads_end) {
+                unsigned long long packed_bins = 0;                          // a byte a bin
+                for (int n = 0; n < 63 && quad < quads_end; ++n, quad += SAMPLE_THREADS) {
+                    float v[4];
+                    scores_of(quad, v);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const uint32_t digits = ordered_key(v[e]) >> shift;
+                        const bool in = quad * 4 + e < end && (shift == 30 || digits >> SAMPLE_DIGIT == found);
+                        packed_bins += in ? 1ull << (8 * (digits & (SAMPLE_BINS - 1))) : 0ull;
+                    }
+                }
+#pragma unroll
+                for (int b = 0; b < SAMPLE_BINS; ++b) bins[b] += (int)(packed_bins >> (8 * b)) & 255;
             }
-            k_index_limit = lo;
+            used = team.sum_bins(bins, totals);
+            // the largest digit from which on k tokens lie
+            int digit = 0;
+            int larger = above;
+#pragma unroll
+            for (int b = SAMPLE_BINS - 1; b > 0; --b)
+                if (digit == 0) {
+                    if (larger + totals[b] >= k) digit = b; else larger += totals[b];
+                }
+            above = larger;
+            k_key |= (uint32_t)digit << shift;
+#pragma unroll
+            for (int b = 0; b < SAMPLE_BINS; ++b) if (b == digit) equal = totals[b];
+        }
+        int wanted = k - above;
+        if (equal > wanted) {              // ties: the first `wanted` of them by token id
+            const int last_digit = k_key & (SAMPLE_BINS - 1);
+            for (int r = 0; r < team.rank; ++r) wanted -= (int)shared.part_bins[used][r][last_digit];
+            // of this CTA's equals the first `wanted` stay (none, or all, where that says so)
+            if (wanted <= 0) k_index_limit = begin;
+            else if (wanted >= (int)shared.part_bins[used][team.rank][last_digit]) k_index_limit = end;
+            else {
+                int lo = begin, hi = end;
+                while (lo < hi) {
+                    const int mid = lo + (hi - lo) / 2;
+                    int count = 0;
+                    for (int quad = first_quad; quad < quads_end && quad * 4 < mid; quad += SAMPLE_THREADS) {
+                        float v[4];
+                        scores_of(quad, v);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) count += quad * 4 + e < mid && ordered_key(v[e]) == k_key;
+                    }
+                    if (team.local_sum(count) >= wanted) hi = mid; else lo = mid + 1;
+                }
+                k_index_limit = lo;
+            }
         }
     }
 #define KEPT_K(key, i) (!use_k || (key) > k_key || ((key) == k_key && (i) < k_index_limit))
@@ -226,25 +311,43 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int vocab,   // logits: 
     const float p_limit = __int_as_float(packed[capacity + row]);
     uint32_t p_key = 0;
     if (p_limit < 1.0f) {
-        float mass = 0.0f;
-        for (int i = begin + tid; i < end; i += SAMPLE_THREADS) {
-            const float s = SCORE(i);
-            if (KEPT_K(ordered_key(s), i)) mass += expf(s);
-        }
-        const float total = team.sum(mass);
-        uint32_t lo = 0, hi = 0xffffffffu;
-        while (lo < hi) {
-            const uint32_t mid = lo + (hi - lo) / 2;
-            float above = 0.0f;
-            for (int i = begin + tid; i < end; i += SAMPLE_THREADS) {
-                const float s = SCORE(i);
-                const uint32_t key = ordered_key(s);
-                if (key > mid && KEPT_K(key, i)) above += expf(s);
+        float above = 0.0f, total = 0.0f;
+        for (int shift = 30; shift >= 0; shift -= SAMPLE_DIGIT) {
+            float bins[SAMPLE_BINS], totals[SAMPLE_BINS];
+#pragma unroll
+            for (int b = 0; b < SAMPLE_BINS; ++b) bins[b] = 0.0f;
+            const uint32_t found = shift == 30 ? 0u : p_key >> (shift + SAMPLE_DIGIT);
+            for (int quad = first_quad; any && quad < quads_end; quad += SAMPLE_THREADS) {
+                float v[4];
+                scores_of(quad, v);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const uint32_t key = ordered_key(v[e]), digits = key >> shift;
+                    if ((shift == 30 || digits >> SAMPLE_DIGIT == found) && quad * 4 + e < end && KEPT_K(key, quad * 4 + e)) {
+                        const float mass = expf(v[e]);
+                        const uint32_t digit = digits & (SAMPLE_BINS - 1);
+#pragma unroll
+                        for (int b = 0; b < SAMPLE_BINS; ++b) bins[b] = __fadd_rn(bins[b], digit == b ? mass : 0.0f);
+                    }
+                }
             }
-            above = team.sum(above);
-            if (__fdiv_rn(above, total) <= p_limit) hi = mid; else lo = mid + 1;
+            team.sum_bins(bins, totals);
+            if (shift == 30) {
+#pragma unroll
+                for (int b = SAMPLE_BINS - 1; b >= 0; --b) total = __fadd_rn(total, totals[b]);
+            }
+            // the smallest digit above all of whose keys no more than top_p lies
+            int digit = shift == 30 ? 3 : SAMPLE_BINS - 1;
+            float larger = above;
+#pragma unroll
+            for (int b = SAMPLE_BINS - 1; b > 0; --b)
+                if (digit == b) {
+                    const float next = __fadd_rn(larger, totals[b]);
+                    if (__fdiv_rn(next, total) <= p_limit) { digit = b - 1; larger = next; }
+                }
+            above = larger;
+            p_key |= (uint32_t)digit << shift;
         }
-        p_key = lo;
     }
 
     // ---- the race
@@ -253,25 +356,42 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int vocab,   // logits: 
     float win = -INFINITY;
     int win_index = 0x7fffffff;
     // a thread takes four consecutive tokens at a time: they share one Philox block
-    for (int quad = begin / 4 + tid; begin < end && quad * 4 < end; quad += SAMPLE_THREADS) {
+    for (int quad = first_quad; any && quad < quads_end; quad += SAMPLE_THREADS) {
+        float v[4];
+        scores_of(quad, v);
+        bool in[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t key = ordered_key(v[e]);
+            in[e] = quad * 4 + e < end && key >= p_key && KEPT_K(key, quad * 4 + e);
+        }
+        if (!(in[0] || in[1] || in[2] || in[3])) continue;
         uint32_t words[4];
         philox4x32_10((uint32_t)quad, draw_lo, draw_hi, 0u, seed_lo, seed_hi, words);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int i = quad * 4 + e;
-            if (i >= end) break;
-            const float s = SCORE(i);
-            const uint32_t key = ordered_key(s);
-            if (key < p_key || !KEPT_K(key, i)) continue;
+            if (!in[e]) continue;
             const float u = __fmul_rn(__fadd_rn((float)(words[e] >> 9), 0.5f), 1.0f / 8388608.0f);
-            const float ratio = __fdiv_rn(expf(s), -logf(u));
-            if (ratio > win) { win = ratio; win_index = i; }
+            const float ratio = __fdiv_rn(expf(v[e]), -logf(u));
+            if (ratio > win) { win = ratio; win_index = quad * 4 + e; }
         }
     }
     team.argmax(win, win_index);
     if (tid == 0 && team.rank == 0) tokens[row] = win_index == 0x7fffffff ? best_index : win_index;
-#undef SCORE
 #undef KEPT_K
+}
+
+template <typename T>
+static cudaError_t launch_sample_rows(const void* logits, long long row_stride, int rows, int vocab, const int* packed,
+                                      int capacity, int* tokens, int pdl, cudaStream_t s) {
+    const long long part = (((long long)vocab + SAMPLE_CTAS - 1) / SAMPLE_CTAS + 3) / 4 * 4;
+    const bool staged = part * 4 <= SAMPLE_STAGED_BYTES;
+    auto kernel = staged ? sample_rows_kernel<T, true> : sample_rows_kernel<T, false>;
+    const int bytes = staged ? (int)part * 4 : 0;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    TvbLaunch launch(dim3(rows * SAMPLE_CTAS), dim3(SAMPLE_THREADS), bytes, s, pdl, SAMPLE_CTAS);
+    return cudaLaunchKernelEx(&launch.config, kernel, (const T*)logits, (int64_t)row_stride, vocab, packed, capacity, tokens);
 }
 
 // packed: int32 [7, capacity], field-major: temperature and top_p as float bits, top_k,
@@ -282,15 +402,9 @@ extern "C" int tvb_sample_rows(const void* logits, long long row_stride, int row
     if (rows <= 0) return 0;
     if (vocab <= 0 || capacity < rows) return TVB_BAD_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
-    TvbLaunch launch(dim3(rows * SAMPLE_CTAS), dim3(SAMPLE_THREADS), 0, s, pdl, SAMPLE_CTAS);
     cudaError_t e;
-    if (dtype == TVB_F32)
-        e = cudaLaunchKernelEx(&launch.config, sample_rows_kernel<float>, (const float*)logits,
-                               (int64_t)row_stride, vocab, packed, capacity, tokens);
-    else if (dtype == TVB_BF16)
-        e = cudaLaunchKernelEx(&launch.config, sample_rows_kernel<bf16>, (const bf16*)logits,
-                               (int64_t)row_stride, vocab, packed, capacity, tokens);
-    else
-        return TVB_BAD_ARGUMENT;
+    if (dtype == TVB_F32) e = launch_sample_rows<float>(logits, row_stride, rows, vocab, packed, capacity, tokens, pdl, s);
+    else if (dtype == TVB_BF16) e = launch_sample_rows<bf16>(logits, row_stride, rows, vocab, packed, capacity, tokens, pdl, s);
+    else return TVB_BAD_ARGUMENT;
     return e == cudaSuccess ? tvb_last_error() : (int)e;
 }
