@@ -22,9 +22,8 @@
 // one of the cluster.  Rows too long for that (more than about 430,000 tokens) read the logits in every pass.
 //
 // Bound by the passes' barriers and compares.  Measured over 151,936 tokens (us; one bit a pass over the logits in L2 /
-// this): 48 rows, half of them greedy, a quarter top-k 50, a quarter top-p 0.95 684 / 140; one row of top-k 50 499 / 53,
-// of top-p 0.95 647 / 77, of both 1,016 / 90; 64 rows of both 1,096 / 325; one greedy row 4.9 / 5.0, 64 greedy rows
-// 11.6 / 17.6 (the shared memory that they do not use leaves two CTAs an SM).
+// this): 48 rows, half of them greedy, a quarter top-k 50, a quarter top-p 0.95 684 / 137; one row of top-k 50 499 / 53,
+// of top-p 0.95 647 / 77, of both 1,016 / 91; 64 rows of both 1,096 / 352; one greedy row 4.9 / 5.4, 64 11.1 / 13.0.
 #include "common.cuh"
 
 #include <cstdint>
@@ -38,6 +37,7 @@ namespace cg = cooperative_groups;
 #define SAMPLE_DIGIT 3          // bits of the threshold that a pass settles
 #define SAMPLE_BINS (1 << SAMPLE_DIGIT)
 #define SAMPLE_STAGED_BYTES (208 * 1024)
+#define SAMPLE_ROWS_AT_ONCE (2 * 148 / SAMPLE_CTAS)
 
 __device__ __forceinline__ uint32_t ordered_key(float f) {
     const uint32_t b = __float_as_uint(f);
@@ -75,6 +75,7 @@ struct RowTeam {
     SampleShared* sh;
     int rank;
     int phase;
+    bool joined;                            // the cluster's CTAs all run: waited for before the first remote store
 
     // count of this CTA alone
     __device__ __forceinline__ int local_sum(int v) {
@@ -165,17 +166,13 @@ struct RowTeam {
     }
 };
 
-// STAGED: the scores stay in shared memory (room for this CTA's part of the row).
-template <typename T, bool STAGED>
-__global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_rows_kernel(const T* logits, int64_t row_stride, int vocab,   // logits: from the kernel before
-                   const int* __restrict__ packed, int capacity, int* __restrict__ tokens) {
-    __shared__ SampleShared shared;
-    extern __shared__ __align__(16) float staged[];
-    RowTeam team{cg::this_cluster(), &shared, (int)(blockIdx.x % SAMPLE_CTAS), 0};
-    cluster_arrive();                       // this CTA runs; waited for before the first remote store
-    pdl_wait();
-    const int row = blockIdx.x / SAMPLE_CTAS, tid = threadIdx.x;
+// The token of one row.  ARGMAX: greedy rows alone, others are left; else STAGED says whether the scores stay in shared
+// memory (room for this CTA's part of the row).
+template <typename T, bool STAGED, bool ARGMAX>
+__device__ __forceinline__ void sample_row(RowTeam& team, SampleShared& shared, float* staged, int row, const T* logits,
+                                           int64_t row_stride, int vocab, const int* __restrict__ packed, int capacity,
+                                           int* __restrict__ tokens) {
+    const int tid = threadIdx.x;
     const T* x = logits + (int64_t)row * row_stride;
     // this CTA's part of the row: whole groups of four tokens (they share a block of noise)
     const int part = ((vocab + SAMPLE_CTAS - 1) / SAMPLE_CTAS + 3) / 4 * 4;
@@ -203,17 +200,21 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int vocab,   // logits: 
     for (int quad = first_quad; any && quad < quads_end; quad += SAMPLE_THREADS) {
         float v[4];
         load_quad(quad, v);
-        if (STAGED && !greedy) reinterpret_cast<float4*>(staged)[quad - begin / 4] = make_float4(v[0], v[1], v[2], v[3]);
+        if (STAGED && !ARGMAX && !greedy) reinterpret_cast<float4*>(staged)[quad - begin / 4] = make_float4(v[0], v[1], v[2], v[3]);
 #pragma unroll
         for (int e = 0; e < 4; ++e)
             if (v[e] > best) { best = v[e]; best_index = 4 * quad + e; }     // (absent is greater than nothing)
     }
-    cluster_wait();
+    if (!team.joined) {
+        cluster_wait();
+        team.joined = true;
+    }
     team.argmax(best, best_index);
-    if (greedy || best_index == 0x7fffffff) {           // the same in every CTA of the row
+    if (ARGMAX || greedy || best_index == 0x7fffffff) {           // the same in every CTA of the row
         if (tid == 0 && team.rank == 0) tokens[row] = best_index == 0x7fffffff ? 0 : best_index;
         return;
     }
+    if constexpr (!ARGMAX) {
     const float row_max = best;
     // Four scores of this thread; a token past the row's end comes as `absent`, whose key is 0.
     auto make_scores = [&](int quad, float* v) {
@@ -379,6 +380,30 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int vocab,   // logits: 
     team.argmax(win, win_index);
     if (tid == 0 && team.rank == 0) tokens[row] = win_index == 0x7fffffff ? best_index : win_index;
 #undef KEPT_K
+    }
+}
+
+// Which rows a launch takes: all of them, the greedy ones, or the others (a cluster then takes several in turn).
+enum SampleRows { ALL_ROWS, GREEDY_ROWS, OTHER_ROWS };
+
+template <typename T, bool STAGED, SampleRows WHICH>
+__global__ void __launch_bounds__(SAMPLE_THREADS, WHICH == GREEDY_ROWS ? 4 : 2)
+sample_rows_kernel(const T* logits, int64_t row_stride, int rows, int vocab,   // logits: from a kernel before
+                   const int* __restrict__ packed, int capacity, int* __restrict__ tokens) {
+    __shared__ SampleShared shared;
+    extern __shared__ __align__(16) float staged[];
+    RowTeam team{cg::this_cluster(), &shared, (int)(blockIdx.x % SAMPLE_CTAS), 0, false};
+    cluster_arrive();                       // this CTA runs; waited for before the first remote store
+    // The launch for the other rows may begin: it looks for rows of its own and waits for this one where it has any.
+    if (WHICH == GREEDY_ROWS) pdl_launch_dependents();
+    if (WHICH != OTHER_ROWS) pdl_wait();
+    for (int row = blockIdx.x / SAMPLE_CTAS; row < rows; row += gridDim.x / SAMPLE_CTAS) {
+        const bool greedy = !(__int_as_float(packed[row]) > 0.0f);
+        if ((WHICH == GREEDY_ROWS && !greedy) || (WHICH == OTHER_ROWS && greedy)) continue;
+        if (WHICH == OTHER_ROWS && !team.joined) pdl_wait();
+        sample_row<T, STAGED, WHICH == GREEDY_ROWS>(team, shared, staged, row, logits, row_stride, vocab, packed, capacity, tokens);
+    }
+    if (!team.joined) cluster_wait();
 }
 
 template <typename T>
@@ -386,12 +411,22 @@ static cudaError_t launch_sample_rows(const void* logits, long long row_stride, 
                                       int capacity, int* tokens, int pdl, cudaStream_t s) {
     const long long part = (((long long)vocab + SAMPLE_CTAS - 1) / SAMPLE_CTAS + 3) / 4 * 4;
     const bool staged = part * 4 <= SAMPLE_STAGED_BYTES;
-    auto kernel = staged ? sample_rows_kernel<T, true> : sample_rows_kernel<T, false>;
     const int bytes = staged ? (int)part * 4 : 0;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    TvbLaunch launch(dim3(rows * SAMPLE_CTAS), dim3(SAMPLE_THREADS), bytes, s, pdl, SAMPLE_CTAS);
-    return cudaLaunchKernelEx(&launch.config, kernel, (const T*)logits, (int64_t)row_stride, vocab, packed, capacity, tokens);
+    auto launch = [&](auto kernel, int clusters, int shared) -> cudaError_t {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
+        if (e != cudaSuccess) return e;
+        TvbLaunch launch(dim3(clusters * SAMPLE_CTAS), dim3(SAMPLE_THREADS), shared, s, pdl, SAMPLE_CTAS);
+        return cudaLaunchKernelEx(&launch.config, kernel, (const T*)logits, (int64_t)row_stride, rows, vocab, packed, capacity, tokens);
+    };
+    // The shared memory leaves room for two CTAs an SM.  Rows beyond those that fit at once would make greedy rows,
+    // which do not use it, wait in line: they get a launch without it (64 greedy rows of 151,936 tokens: 17.6 us in one
+    // launch).
+    if (rows <= SAMPLE_ROWS_AT_ONCE || !staged)
+        return staged ? launch(sample_rows_kernel<T, true, ALL_ROWS>, rows, bytes)
+                      : launch(sample_rows_kernel<T, false, ALL_ROWS>, rows, bytes);
+    const cudaError_t e = launch(sample_rows_kernel<T, false, GREEDY_ROWS>, rows, 0);
+    pdl = 1;                                 // whatever the first launch was: the second waits for it by itself
+    return e != cudaSuccess ? e : launch(sample_rows_kernel<T, true, OTHER_ROWS>, SAMPLE_ROWS_AT_ONCE, bytes);
 }
 
 // packed: int32 [7, capacity], field-major: temperature and top_p as float bits, top_k,
