@@ -158,6 +158,7 @@ class StepRunner:
         self.tensor_memory_tiles = self.dtype == torch.bfloat16 and len(blocks) > 0 and all(
             getattr(block, "takes_tensor_memory_tiles", lambda page: False)(page_size)
             for block in blocks)
+        self.small_context = max((getattr(getattr(block, "mixer", None), "small_context", 0) for block in blocks), default=0)
 
     # ------------------------------------------------------------- sizing
     @staticmethod
@@ -234,7 +235,7 @@ class StepRunner:
         if tiled:
             tc_lists, tile_lists, single_runs = attention_ops.prefill_tiles(
                 counts, [p.start for p in plan.entries], tensor_memory=self.tensor_memory_tiles,
-                singles_apart=True)
+                singles_apart=True, small_context=self.small_context)
         else:
             tc_lists, tile_lists, single_runs = ([], [], []), ([], [], []), ()
         sizes = [tokens, tokens, tokens, wanted, rows, rows + 1]

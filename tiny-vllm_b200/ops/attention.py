@@ -18,6 +18,7 @@ max(0, p - window + 1) to p through the block table.
 
 from __future__ import annotations
 
+import math
 import os
 
 import torch
@@ -115,24 +116,32 @@ def far_plan(rows: int, mixer, page_size: int, max_context: int):
     return None
 
 
-# tiles with fewer tokens than this go to the 64-row kernel: a 128-row tensor-memory tile is mostly
-# empty for them
+# An entry with fewer tokens than this does not ask for a launch of the 128-row kernel (a tile of tensor memory is
+# mostly empty for it); where the step has such tiles anyway it joins them, as do the last tokens of a longer
+# entry: an item more on some SM costs less than a launch of another kernel beside (28 layers of 16 q / 8 kv
+# heads: a step of 2,060 tokens took 3.8 ms with its last 12 tokens in the kernel for single tokens, 3.2 with them in tiles).
 TC_MIN_TILE_TOKENS = 32
 
 
-def prefill_tiles(counts, starts=None, *, tensor_memory: bool = False, singles_apart: bool = False):
+def prefill_tiles(counts, starts=None, *, tensor_memory: bool = False, singles_apart: bool = False,
+                  small_context: int = 0):
     """Cut every entry of a step into tiles of consecutive tokens.
 
     Returns two triples of lists (row, first flat token, count) and a list of runs: tiles of up to
     128 tokens for the tcgen05 kernel, the longest context first; tiles of up to 64 tokens for the
     mma.sync kernel; and, with ``singles_apart``, (first flat token, count) of every run of
     consecutive tokens that are attended one by one: single-token entries (decoded tokens beside
-    prompt portions) and, with ``tensor_memory``, the rests of entries too short for a tile.  Without
-    ``tensor_memory`` nothing is in the first set; with it only the short rests of entries are in
-    the second.  ``starts``: tokens each entry has in the cache before the step."""
+    prompt portions) and, with ``tensor_memory``, the entries of a step without one long enough for a tile.  Without
+    ``tensor_memory`` nothing is in the first set; with it (and without ``singles_apart``) only the short
+    rests of entries are in the second.  ``starts``: tokens each entry has in the cache before the step.
+    ``small_context``: a step whose prompt entries all end within so many keys is cut for the 64-row kernel."""
     small = kernels.attention_prefill_tile_tokens()
     large = kernels.attention_prefill_tc_tile_tokens() if tensor_memory else 0
     starts = starts if starts is not None else [0] * len(counts)
+    if all(count == 1 or start + count <= small_context for start, count in zip(starts, counts)):
+        large = 0
+    # with tiles of tensor memory in the step, every prompt entry is cut into them to its end
+    whole = large > 0 and singles_apart and max(counts, default=0) >= TC_MIN_TILE_TOKENS
     big, ends = ([], [], []), []
     rest = ([], [], [])
     runs: list[list[int]] = []
@@ -146,14 +155,14 @@ def prefill_tiles(counts, starts=None, *, tensor_memory: bool = False, singles_a
             cursor += 1
             continue
         done = 0
-        if tensor_memory:
-            while count - done >= TC_MIN_TILE_TOKENS:
+        if large > 0:
+            while count - done >= (1 if whole else TC_MIN_TILE_TOKENS):
                 size = min(large, count - done)
                 big[0].append(row), big[1].append(cursor + done), big[2].append(size)
                 ends.append(starts[row] + done + size)
                 done += size
             if singles_apart and done < count:
-                # the short rest of an entry: token by token like decoded tokens (a 64-row tile for a
+                # an entry too short for a tile: token by token like decoded tokens (a 64-row tile for a
                 # few tokens walks a long context alone: 75 us at 2,048 keys, whatever their number)
                 if runs and runs[-1][0] + runs[-1][1] == cursor + done:
                     runs[-1][1] += count - done
@@ -336,8 +345,9 @@ def windowed_attention(ctx, mixer, projected: torch.Tensor, at: int, run: int, o
                  gate_per_head=mixer.gate == "head", slopes=mixer.slopes, sinks=mixer.sinks,
                  bias_table=bias_table, segment=segment, softcap=getattr(mixer, "softcap", None))
     if not (segment and mixer.window) and windowed_on_tensor_cores(mixer, projected, q_at, g_at, out):
-        # bfloat16: prompt portions in tiles of 64 tokens, single tokens (decoded ones, whose keys are in the
-        # cache by now) one CTA per kv head and chunk of keys
+        # bfloat16: prompt portions in tiles of 128 tokens on tcgen05 where every mixer of the model takes them, else of
+        # 64 on mma.sync; single tokens (decoded ones, and the short rests of portions beside tiles of 128, whose
+        # keys are in the cache by now) one CTA per kv head and chunk of keys
         def singles(part):
             need = kernels.attention_tiles_singles_floats(
                 part.stop - part.start, mixer.num_heads, mixer.value_dim, segment or mixer.window, mixer.keep_first,
@@ -351,6 +361,17 @@ def windowed_attention(ctx, mixer, projected: torch.Tensor, at: int, run: int, o
             singles(slice(0, ctx.num_tokens))
             return
         if ctx.tile_row is not None:
+            if ctx.tile_tc_row is not None and ctx.tile_tc_row.shape[0] > 0:
+                # the step's tile lists were cut for the tcgen05 kernel: every mixer of the model takes it
+                plain = {name: value for name, value in heads.items() if name not in ("slopes", "softcap")}
+                aligned = out
+                if out.stride(0) % 8 or out.data_ptr() % 16:
+                    aligned = torch.empty(out.shape, dtype=out.dtype, device=out.device)
+                kernels.attention_prefill_tc_extras(
+                    queries, keys, values, ctx.block_tables[group], ctx.positions, ctx.tile_tc_row, ctx.tile_tc_first,
+                    ctx.tile_tc_count, **plain, out=aligned, gate=gate)
+                if aligned is not out:
+                    out.copy_(aligned)
             if ctx.tile_row.shape[0] > 0:
                 kernels.attention_tiles(queries, keys, values, ctx.block_tables[group], ctx.positions, ctx.tile_row,
                                         ctx.tile_first, ctx.tile_count, **heads, out=out, gate=gate)
@@ -367,6 +388,20 @@ def windowed_attention(ctx, mixer, projected: torch.Tensor, at: int, run: int, o
         value_dim=mixer.value_dim, window=mixer.window, keep_first=mixer.keep_first, scale=mixer.scale,
         gate=gate, gate_per_head=mixer.gate == "head", slopes=mixer.slopes, sinks=mixer.sinks, out=out,
         scratch=scratch, max_chunks=ctx.split_chunks, bias_table=bias_table, segment=segment, softcap=getattr(mixer, "softcap", None))
+
+
+def windowed_takes_tensor_memory_tiles(mixer, page_size: int) -> bool:
+    """Whether the tcgen05 kernel takes the prompt portions of a mixer of :func:`windowed_attention`: keys and values of 128
+    in caches of their own, no slopes, no cap on the scores, a learned bias of so many distances at most, a window or
+    segments but not both.  Measured at 16 q / 8 kv heads (us a layer, mma.sync kernel / this): 2,048 tokens, window 1,024 with 4
+    kept keys 131 / 41; prompts of 1,501, 1,126 and 751 tokens in segments of 1,024 with a bias, a sink and a gate
+    181 / 71; one of 300 tokens 27 / 14 and 37 / 19, one of 33 9 / 10 and 15 / 14."""
+    if (mixer.key_dim, mixer.value_dim) != (128, 128) or mixer.softcap is not None \
+            or mixer.distance_slope_exponent is not None or (mixer.segment and mixer.window) or not TENSOR_CORE_WINDOWS:
+        return False
+    if mixer.distance_table is not None and math.ceil(mixer.distance_table[1]) + 1 > kernels.attention_prefill_tc_bias_rows():
+        return False
+    return kernels.attention_prefill_tc_supports(128, mixer.num_heads, mixer.num_kv_heads, page_size)
 
 
 def latent_attention(ctx, mixer, projected: torch.Tensor, run: int) -> torch.Tensor:

@@ -2142,6 +2142,69 @@ def attention_prefill_tc(q: torch.Tensor, q_token_stride: int, key_cache: torch.
     return out
 
 
+_prefill_tc_bias_rows: int | None = None
+
+
+def attention_prefill_tc_bias_rows() -> int:
+    """Rows (distances) a learned bias may have in :func:`attention_prefill_tc_extras`."""
+    global _prefill_tc_bias_rows
+    if _prefill_tc_bias_rows is None:
+        _prefill_tc_bias_rows = _fn("attention_prefill_tc", "tvb_attention_prefill_tc_bias_rows", [])()
+    return _prefill_tc_bias_rows
+
+
+def attention_prefill_tc_extras(q: torch.Tensor, key_cache: torch.Tensor, value_cache: torch.Tensor,
+                                block_tables: torch.Tensor, positions: torch.Tensor, tile_row: torch.Tensor,
+                                tile_first: torch.Tensor, tile_count: torch.Tensor, *, num_q: int, num_kv: int,
+                                key_dim: int, value_dim: int, window: int | None, keep_first: int, scale: float,
+                                out: torch.Tensor, gate: torch.Tensor | None = None, gate_per_head: bool = False,
+                                sinks: torch.Tensor | None = None, bias_table: torch.Tensor | None = None,
+                                segment: int | None = None) -> torch.Tensor:
+    """:func:`attention_tiles` (without slopes and softcap) on the tcgen05 tensor cores: keys and values of 128, tiles
+    of up to 128 tokens, the longest context first.  ``out`` has 16-byte aligned rows; the gate's may lie anywhere."""
+    _need_cuda(q, key_cache, value_cache, block_tables, positions, tile_row, tile_first, tile_count, out, gate, sinks,
+               bias_table)
+    who = "attention_prefill_tc_extras"
+    _tiles_table(who, bias_table, segment, window, num_q)
+    if (key_dim, value_dim) != (128, 128) or not attention_prefill_tc_supports(128, num_q, num_kv, key_cache.shape[2]):
+        raise KernelError(f"{who} does not take heads of {key_dim} and {value_dim}, {num_q}/{num_kv} of them, pages of "
+                          f"{key_cache.shape[2]}")
+    if bias_table is not None and bias_table.shape[0] > attention_prefill_tc_bias_rows():
+        raise KernelError(f"{who}: a bias table has up to {attention_prefill_tc_bias_rows()} rows")
+    shape = (key_cache.shape[0], num_kv, key_cache.shape[2], 128)
+    if q.dtype != torch.bfloat16 or any(c.dtype != torch.bfloat16 or c.shape != shape or not c.is_contiguous()
+                                        for c in (key_cache, value_cache)):
+        raise KernelError(f"{who}: bfloat16, with contiguous caches [pages, num_kv, page_size, 128]")
+    tokens, tiles = positions.shape[0], tile_row.shape[0]
+    if q.dim() != 2 or q.stride(1) != 1 or q.stride(0) % 8 or q.data_ptr() % 16 or q.shape[1] < num_q * 128:
+        raise KernelError(f"{who}: q must be [tokens, >= num_q * 128] with 16-byte aligned rows")
+    if out.shape != (tokens, num_q * 128) or out.dtype != torch.bfloat16 or out.stride(1) != 1 or out.stride(0) % 8 \
+            or out.data_ptr() % 16:
+        raise KernelError(f"{who}: out must be bfloat16 [tokens, num_q * 128] with 16-byte aligned rows")
+    if gate is not None and (gate.shape != (tokens, num_q if gate_per_head else num_q * 128) or gate.stride(1) != 1
+                             or gate.dtype != torch.bfloat16):
+        raise KernelError(f"{who}: the gate is bfloat16, one number a value or a head, with contiguous rows")
+    if sinks is not None and (sinks.dtype != torch.float32 or sinks.shape != (num_q,) or not sinks.is_contiguous()):
+        raise KernelError(f"{who}: sinks must be contiguous float32 [num_q]")
+    for t in (block_tables, positions, tile_row, tile_first, tile_count):
+        if t.dtype != torch.int32 or not t.is_contiguous():
+            raise KernelError(f"{who}: index tensors must be contiguous int32")
+    fn = _fn("attention_prefill_tc", "tvb_attention_prefill_tc_extras",
+             [c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p,
+              c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p]
+             + [c_int] * 8 + [c_float, c_int, c_void_p])
+    global _attention_tc_unchecked
+    _check(fn(q.data_ptr(), q.stride(0), tokens, key_cache.data_ptr(), value_cache.data_ptr(), key_cache.shape[0],
+              block_tables.data_ptr(), block_tables.shape[1], positions.data_ptr(), tile_row.data_ptr(),
+              tile_first.data_ptr(), tile_count.data_ptr(), tiles, out.data_ptr(), out.stride(0), _ptr(gate),
+              0 if gate is None else gate.stride(0), 1 if gate_per_head else 0, _ptr(sinks), _ptr(bias_table),
+              0 if bias_table is None else bias_table.shape[0], num_q, num_kv, 128, key_cache.shape[2], window or 0,
+              keep_first if window else 0, segment or 0, scale, _pdl("prefill"), _stream()), who)
+    _attention_tc_unchecked = True
+    _guarded_counts[1] += 1
+    return out
+
+
 def attention_prefill_tc_status() -> int:
     """0, or which bounded wait of an attention_prefill_tc launch gave up since the last call.
     Synchronises the device; reading clears the record."""

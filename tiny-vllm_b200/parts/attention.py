@@ -341,7 +341,11 @@ class WindowedAttention(Part):
         return KVNeed(self.num_kv_heads, self.key_dim, self.window, self.value_dim, self.keep_first)
 
     def takes_tensor_memory_tiles(self, page_size: int) -> bool:
-        return False
+        return attention_ops.windowed_takes_tensor_memory_tiles(self, page_size)
+
+    # keys up to which the 64-row kernel is the faster one for prompt portions (us a layer at 16 q / 8 kv heads, 64-row /
+    # 128-row: 33 tokens 9.3 / 10.5, 100 tokens 13.8 / 10.3)
+    small_context = 64
 
     def scratch_floats(self, rows: int, chunks: int) -> int:
         """float32 scratch for ``rows`` single tokens whose keys span ``chunks`` chunks: what the row
