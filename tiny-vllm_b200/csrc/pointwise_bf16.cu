@@ -5,23 +5,48 @@
 // :153-211, :274-285; tinyvllm/kernels/kv_store.cu:26-90).
 #include "common.cuh"
 
+// Eight weights from p on, as 16-byte words (p on such a boundary).
+__device__ __forceinline__ void load_weights8(const float* p, float* w) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+    w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+}
+__device__ __forceinline__ void load_weights8(const bf16* p, float* w) {
+    unpack_bf16x8(*reinterpret_cast<const uint4*>(p), w);
+}
+// ... and at any address
+template <typename W> __device__ __forceinline__ void load_weights8(const W* p, bool in_words, float* w) {
+    if (in_words) load_weights8(p, w);
+    else
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = to_float<W>(p[e]);
+}
+
 // -------------------------------------------------------------------- RMSNorm
 // TPR threads share a row (32: one warp, 8 rows a CTA; 64, 128; 256: the whole CTA).  A thread holds up to
-// 4 words of 8 values.  `x` and `residual` come from the kernel before: coherent loads.
+// 4 words of 8 values.  `x` and `residual` come from the kernel before: coherent loads.  The weights do not:
+// they are read before the wait for it, in 16-byte words where they lie on such a boundary (read one by one behind the
+// row's sum, 32 bytes from lane to lane, they made it 5.8 us for 2,048 rows of 1,024 instead of 4.2, and 51 for 8,192 of 4,096 instead of 42).
 #define NORM_WORDS 4
 
 template <int TPR, typename W>
 __global__ void __launch_bounds__(256)
 rms_norm_bf16_kernel(const bf16* x, const bf16* residual, const W* __restrict__ weight,
                      bf16* __restrict__ y, bf16* __restrict__ residual_out,
-                     const int* __restrict__ gather, int rows, int width, float eps) {
+                     const int* __restrict__ gather, int rows, int width, float eps, int weight_words) {
     __shared__ float scratch[32];
     __shared__ float row_parts[8];
-    pdl_wait();
-    pdl_launch_dependents();
     const int rows_per_cta = 256 / TPR;
     const int out_row = blockIdx.x * rows_per_cta + threadIdx.x / TPR;
     const int lane = threadIdx.x % TPR;
+    float weights[NORM_WORDS][8];
+#pragma unroll
+    for (int i = 0; i < NORM_WORDS; ++i) {
+        const int at = (lane + i * TPR) * 8;
+        if (at < width) load_weights8<W>(weight + at, weight_words, weights[i]);
+    }
+    pdl_wait();
+    pdl_launch_dependents();
     const bool live = out_row < rows;
     const int in_row = live ? (gather ? gather[out_row] : out_row) : 0;
     const bf16* xr = x + (int64_t)in_row * width;
@@ -78,7 +103,7 @@ rms_norm_bf16_kernel(const bf16* x, const bf16* residual, const W* __restrict__ 
             float out[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-                out[e] = __fmul_rn(round_to<bf16>(__fmul_rn(values[i][e], inverse_rms)), to_float<W>(weight[at + e]));
+                out[e] = __fmul_rn(round_to<bf16>(__fmul_rn(values[i][e], inverse_rms)), weights[i][e]);
             *reinterpret_cast<uint4*>(y + (int64_t)out_row * width + at) = pack_bf16x8(out);
         }
     }
@@ -102,7 +127,7 @@ extern "C" int tvb_rms_norm_bf16(const void* x, const void* residual, const void
 #define NORM_LAUNCH(TPR, WT)                                                                          \
     e = cudaLaunchKernelEx(&launch.config, rms_norm_bf16_kernel<TPR, WT>, (const bf16*)x,             \
                            (const bf16*)residual, (const WT*)weight, (bf16*)y, (bf16*)residual_out,   \
-                           gather, rows, width, eps)
+                           gather, rows, width, eps, (int)(((uintptr_t)weight & 15) == 0))
 #define NORM_BY_TPR(WT)                                        \
     do {                                                       \
         if (tpr == 32) NORM_LAUNCH(32, WT);                    \
