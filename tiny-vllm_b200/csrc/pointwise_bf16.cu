@@ -191,7 +191,7 @@ qk_norm_rope_store_bf16_kernel(bf16* __restrict__ qkv, const W* __restrict__ q_w
     constexpr int GROUPS = 32 / LANES;
     constexpr int BATCH = 4;
     const int heads = num_q + 2 * num_kv;
-    const int token = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (token >= tokens) return;                 // the whole warp
     const int lane = threadIdx.x & 31;
     const int group = lane / LANES, l = lane % LANES;
@@ -318,7 +318,10 @@ extern "C" int tvb_qk_norm_rope_store_bf16(void* qkv, const void* q_weight, cons
     if (!tvb_qk_norm_rope_store_bf16_supports(head_dim) || num_q <= 0 || num_kv < 0 || (slots && page_size <= 0))
         return TVB_BAD_ARGUMENT;
     if (head_dim % 8 || ((num_q + 2 * num_kv) * head_dim) % 8) return TVB_BAD_ARGUMENT;
-    const int64_t blocks = ((int64_t)tokens + 7) / 8;         // a warp per token, eight to a block
+    // a warp per token, eight to a block; from 1,024 tokens on two, so that the last blocks even out over the SMs
+    // (16 q / 8 kv heads, 4,000 tokens 13.9 us with eight, 13.2 with two; 32 / 8, 8,192 tokens 44.3 and 42.3)
+    const int together = tokens >= 1024 ? 2 : 8;
+    const int64_t blocks = ((int64_t)tokens + together - 1) / together;
     cudaStream_t s = (cudaStream_t)stream;
     // With few tokens (a warp each) the heads of a token are shared out over more CTAs: a batch of
     // heads (four per group of lanes) per CTA along y while the grid stays within one CTA an SM
@@ -329,7 +332,7 @@ extern "C" int tvb_qk_norm_rope_store_bf16(void* qkv, const void* q_weight, cons
     int along_y = (num_q + 2 * num_kv + batch_heads - 1) / batch_heads;
     const long long room = (long long)tvb_sm_count_pointwise() / (blocks > 0 ? blocks : 1);
     if (along_y > room) along_y = room < 1 ? 1 : (int)room;
-    TvbLaunch launch(dim3((unsigned)blocks, (unsigned)along_y), dim3(256), 0, s, pdl);
+    TvbLaunch launch(dim3((unsigned)blocks, (unsigned)along_y), dim3(together * 32), 0, s, pdl);
     cudaError_t launched = cudaSuccess;
 #define QK_LAUNCH(D, WT)                                                                                   \
     launched = cudaLaunchKernelEx(&launch.config, qk_norm_rope_store_bf16_kernel<D, WT>,                   \
