@@ -394,9 +394,10 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int rows, int vocab,   /
     extern __shared__ __align__(16) float staged[];
     RowTeam team{cg::this_cluster(), &shared, (int)(blockIdx.x % SAMPLE_CTAS), 0, false};
     cluster_arrive();                       // this CTA runs; waited for before the first remote store
-    // The launch for the other rows may begin: it looks for rows of its own and waits for this one where it has any.
-    if (WHICH == GREEDY_ROWS) pdl_launch_dependents();
     if (WHICH != OTHER_ROWS) pdl_wait();
+    // What both launches read is there: the one for the other rows may begin, to see whether it has any, and waits
+    // for this one where it does.
+    if (WHICH == GREEDY_ROWS) pdl_launch_dependents();
     for (int row = blockIdx.x / SAMPLE_CTAS; row < rows; row += gridDim.x / SAMPLE_CTAS) {
         const bool greedy = !(__int_as_float(packed[row]) > 0.0f);
         if ((WHICH == GREEDY_ROWS && !greedy) || (WHICH == OTHER_ROWS && greedy)) continue;
