@@ -253,7 +253,7 @@ class StepRunner:
         row_starts = view(5)
         for r, (entry, planned) in enumerate(zip(entries, plan.entries)):
             n = counts[r]
-            view(0)[cursor:cursor + n] = entry.tokens
+            view(0)[cursor:cursor + n] = np.fromiter(entry.tokens, np.int32, n)
             view(1)[cursor:cursor + n] = np.arange(planned.start, planned.start + n, dtype=np.int32)
             view(2)[cursor:cursor + n] = r
             for place in entry.want:
@@ -262,8 +262,14 @@ class StepRunner:
             view(4)[r] = planned.state_slot
             row_starts[r] = cursor
             for g in range(groups):
-                view(6 + 2 * g)[cursor:cursor + n] = planned.slots[g]
                 table = planned.tables[g]
+                if n == 1:
+                    view(6 + 2 * g)[cursor] = planned.slots[g][0]
+                else:                          # planned.slots[g], from the pages instead of token by token
+                    size, at = self.manager.page_size, planned.start
+                    pages = np.array(table[at // size:(at + n - 1) // size + 1], dtype=np.int32)
+                    slots = (pages[:, None] * size + np.arange(size, dtype=np.int32)).reshape(-1)
+                    view(6 + 2 * g)[cursor:cursor + n] = slots[at % size:at % size + n]
                 view(7 + 2 * g)[r * blocks[g]:r * blocks[g] + len(table)] = table
             max_position = max(max_position, planned.start + n - 1)
             cursor += n
