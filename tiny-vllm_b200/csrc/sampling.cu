@@ -23,7 +23,7 @@
 //
 // Bound by the passes' barriers and compares.  Measured over 151,936 tokens (us; one bit a pass over the logits in L2 /
 // this): 48 rows, half of them greedy, a quarter top-k 50, a quarter top-p 0.95 684 / 137; one row of top-k 50 499 / 53,
-// of top-p 0.95 647 / 77, of both 1,016 / 91; 64 rows of both 1,096 / 352; one greedy row 4.9 / 5.4, 64 11.1 / 13.0.
+// of top-p 0.95 647 / 77, of both 1,016 / 91; 64 rows of both 1,096 / 352; one greedy row 4.1 / 4.3, 64 10.6 / 12.5.
 #include "common.cuh"
 
 #include <cstdint>
@@ -196,14 +196,25 @@ __device__ __forceinline__ void sample_row(RowTeam& team, SampleShared& shared, 
     int best_index = 0x7fffffff;
     const float temp = __int_as_float(packed[row]);
     const bool greedy = !(temp > 0.0f);
-#pragma unroll 5
-    for (int quad = first_quad; any && quad < quads_end; quad += SAMPLE_THREADS) {
-        float v[4];
-        load_quad(quad, v);
+    auto meet = [&](int quad, const float* v) {
         if (STAGED && !ARGMAX && !greedy) reinterpret_cast<float4*>(staged)[quad - begin / 4] = make_float4(v[0], v[1], v[2], v[3]);
 #pragma unroll
         for (int e = 0; e < 4; ++e)
             if (v[e] > best) { best = v[e]; best_index = 4 * quad + e; }     // (absent is greater than nothing)
+    };
+    // whole words without a condition between their loads, so that several are in flight; then what is left
+    int quad = first_quad;
+    if (any && wide)
+#pragma unroll 5
+        for (; quad < end / 4; quad += SAMPLE_THREADS) {
+            const float4 f = reinterpret_cast<const float4*>(x)[quad];
+            const float v[4] = {f.x, f.y, f.z, f.w};
+            meet(quad, v);
+        }
+    for (; any && quad < quads_end; quad += SAMPLE_THREADS) {
+        float v[4];
+        load_quad(quad, v);
+        meet(quad, v);
     }
     if (!team.joined) {
         cluster_wait();
