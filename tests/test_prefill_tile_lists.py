@@ -12,10 +12,10 @@ def sizes(monkeypatch):
     monkeypatch.setattr(kernels, "attention_prefill_tc_tile_tokens", lambda: 128)
 
 
-def test_short_rests_and_entries_join_the_tiles_of_a_step_that_has_some():
+def test_short_rests_are_attended_one_by_one():
     big, rest, runs = prefill_tiles([140, 1, 9, 1], [0, 700, 300, 5], tensor_memory=True, singles_apart=True)
-    assert big == ([2, 0, 0], [141, 128, 0], [9, 12, 128])              # the longest context first
-    assert rest == ([], [], []) and runs == ((140, 1), (150, 1))
+    assert big == ([0], [0], [128])
+    assert rest == ([], [], []) and runs == ((128, 23),)
 
 
 def test_a_step_of_short_entries_asks_for_no_tiles():
@@ -23,8 +23,33 @@ def test_a_step_of_short_entries_asks_for_no_tiles():
         ([], [], []), ([], [], []), ((0, 40),))
 
 
-@pytest.mark.parametrize("counts,starts,small", [([40, 20], [0, 0], True), ([40, 1], [24, 900], True), ([40], [25], False),
-                                                 ([9, 65], [0, 0], False)])
-def test_small_contexts_stay_with_the_64_row_kernel(counts, starts, small):
-    big, rest, _ = prefill_tiles(counts, starts, tensor_memory=True, singles_apart=True, small_context=64)
-    assert (len(big[0]) == 0) == small and (len(rest[0]) > 0) == small
+@pytest.mark.parametrize("counts,starts,big_rows,rest_rows", [
+    ([40, 20], [0, 0], [], [0, 1]), ([40, 1], [24, 900], [], [0]), ([40], [25], [0], []), ([9, 65], [0, 0], [1], [0]),
+    ([300, 31, 32], [0, 900, 900], [2, 0, 0, 0], [1])])
+def test_entries_go_whole_to_one_of_the_two_kernels(counts, starts, big_rows, rest_rows):
+    big, rest, runs = prefill_tiles(counts, starts, tensor_memory=True, singles_apart=True, small_context=64)
+    assert (big[0], rest[0]) == (big_rows, rest_rows)
+    assert sum(big[2]) + sum(rest[2]) == sum(counts) - counts.count(1) == sum(counts) - sum(n for _, n in runs)
+
+
+def cut_of(row, counts, starts, small_context):
+    """What becomes of entry ``row``: (kernel, first token within the entry, tokens) of every piece, token by token where
+    tokens go one by one."""
+    big, rest, runs = prefill_tiles(counts, starts, tensor_memory=True, singles_apart=True, small_context=small_context)
+    at = sum(counts[:row])
+    pieces = [(kind, first - at, count) for kind, lists in (("128", big), ("64", rest))
+              for r, first, count in zip(*lists) if r == row]
+    for first, count in runs:
+        pieces += [("one", t - at, 1) for t in range(max(first, at), min(first + count, at + counts[row]))]
+    return sorted(pieces)
+
+
+@pytest.mark.parametrize("small_context", [0, 64])
+@pytest.mark.parametrize("count,start", [(1, 0), (1, 500), (2, 0), (9, 300), (31, 0), (32, 0), (40, 24), (40, 25), (140, 0), (160, 700)])
+def test_an_entry_is_cut_the_same_beside_any_other(count, start, small_context):
+    alone = cut_of(0, [count], [start], small_context)
+    assert sum(n for _, _, n in alone) == count
+    for other, at in ((1, 0), (1, 900), (9, 0), (31, 40), (33, 0), (40, 24), (500, 0), (500, 800)):
+        assert cut_of(0, [count, other], [start, at], small_context) == alone
+        assert cut_of(1, [other, count], [at, start], small_context) == alone
+        assert cut_of(1, [other, count, other], [at, start, at], small_context) == alone

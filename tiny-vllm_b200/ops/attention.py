@@ -8,7 +8,7 @@ max(0, p - window + 1) to p through the block table.
   (``attention_decode``): norm, rotation, cache write and attention split over a cluster.
 * bfloat16 prompt portions, head size 128: ``qk_norm_rope_store``, then tiles of up to 128
   tokens on the tcgen05 kernel (``attention_prefill_tc``: S, P and O in tensor memory); the
-  decoded tokens of the same step, and all tokens of a step whose portions are shorter than 32, are
+  decoded tokens of the same step and the rests of portions shorter than 32 tokens are
   attended token by token by ``attention_decode`` (their keys are in the cache by then).
 * bfloat16 prompt portions, head size 64 (or pages the tcgen05 kernel does not take): tiles of
   64 tokens on the mma.sync kernel (``attention_prefill``).
@@ -116,10 +116,7 @@ def far_plan(rows: int, mixer, page_size: int, max_context: int):
     return None
 
 
-# An entry with fewer tokens than this does not ask for a launch of the 128-row kernel (a tile of tensor memory is
-# mostly empty for it); where the step has such tiles anyway it joins them, as do the last tokens of a longer
-# entry: an item more on some SM costs less than a launch of another kernel beside (28 layers of 16 q / 8 kv
-# heads: a step of 2,060 tokens took 3.8 ms with its last 12 tokens in the kernel for single tokens, 3.2 with them in tiles).
+# tiles with fewer tokens than this stay off the 128-row kernel: a tile of tensor memory is mostly empty for them
 TC_MIN_TILE_TOKENS = 32
 
 
@@ -131,17 +128,17 @@ def prefill_tiles(counts, starts=None, *, tensor_memory: bool = False, singles_a
     128 tokens for the tcgen05 kernel, the longest context first; tiles of up to 64 tokens for the
     mma.sync kernel; and, with ``singles_apart``, (first flat token, count) of every run of
     consecutive tokens that are attended one by one: single-token entries (decoded tokens beside
-    prompt portions) and, with ``tensor_memory``, the entries of a step without one long enough for a tile.  Without
-    ``tensor_memory`` nothing is in the first set; with it (and without ``singles_apart``) only the short
-    rests of entries are in the second.  ``starts``: tokens each entry has in the cache before the step.
-    ``small_context``: a step whose prompt entries all end within so many keys is cut for the 64-row kernel."""
+    prompt portions) and, with ``tensor_memory``, the rests of entries too short for a tile.  Without
+    ``tensor_memory`` nothing is in the first set; with it only the short rests of entries are in
+    the second.  ``starts``: tokens each entry has in the cache before the step.
+
+    ``small_context`` > 0 (with ``tensor_memory``): an entry goes to one kernel whole, its short rest too: to
+    the 128-row one if it has TC_MIN_TILE_TOKENS tokens and ends beyond so many keys, else to the 64-row one.
+
+    How an entry is cut depends on that entry alone, not on what else is in the step."""
     small = kernels.attention_prefill_tile_tokens()
     large = kernels.attention_prefill_tc_tile_tokens() if tensor_memory else 0
     starts = starts if starts is not None else [0] * len(counts)
-    if all(count == 1 or start + count <= small_context for start, count in zip(starts, counts)):
-        large = 0
-    # with tiles of tensor memory in the step, every prompt entry is cut into them to its end
-    whole = large > 0 and singles_apart and max(counts, default=0) >= TC_MIN_TILE_TOKENS
     big, ends = ([], [], []), []
     rest = ([], [], [])
     runs: list[list[int]] = []
@@ -155,14 +152,15 @@ def prefill_tiles(counts, starts=None, *, tensor_memory: bool = False, singles_a
             cursor += 1
             continue
         done = 0
-        if large > 0:
+        whole = small_context > 0
+        if large > 0 and not (whole and (count < TC_MIN_TILE_TOKENS or starts[row] + count <= small_context)):
             while count - done >= (1 if whole else TC_MIN_TILE_TOKENS):
                 size = min(large, count - done)
                 big[0].append(row), big[1].append(cursor + done), big[2].append(size)
                 ends.append(starts[row] + done + size)
                 done += size
             if singles_apart and done < count:
-                # an entry too short for a tile: token by token like decoded tokens (a 64-row tile for a
+                # the short rest of an entry: token by token like decoded tokens (a 64-row tile for a
                 # few tokens walks a long context alone: 75 us at 2,048 keys, whatever their number)
                 if runs and runs[-1][0] + runs[-1][1] == cursor + done:
                     runs[-1][1] += count - done
@@ -345,9 +343,9 @@ def windowed_attention(ctx, mixer, projected: torch.Tensor, at: int, run: int, o
                  gate_per_head=mixer.gate == "head", slopes=mixer.slopes, sinks=mixer.sinks,
                  bias_table=bias_table, segment=segment, softcap=getattr(mixer, "softcap", None))
     if not (segment and mixer.window) and windowed_on_tensor_cores(mixer, projected, q_at, g_at, out):
-        # bfloat16: prompt portions in tiles of 128 tokens on tcgen05 where every mixer of the model takes them, else of
-        # 64 on mma.sync; single tokens (decoded ones, and the short rests of portions beside tiles of 128, whose
-        # keys are in the cache by now) one CTA per kv head and chunk of keys
+        # bfloat16: prompt portions in tiles of 128 tokens on tcgen05 where every mixer of the model takes them, but for
+        # portions of less than 32 tokens or that end within `small_context` keys; those, and all portions of
+        # other models, in tiles of 64 on mma.sync; decoded tokens one CTA per kv head and chunk of keys
         def singles(part):
             need = kernels.attention_tiles_singles_floats(
                 part.stop - part.start, mixer.num_heads, mixer.value_dim, segment or mixer.window, mixer.keep_first,
