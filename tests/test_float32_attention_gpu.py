@@ -53,3 +53,44 @@ def test_a_later_token_that_is_not_finite_touches_no_earlier_one():
         case[cache][page, :, at % 16] = value
     after = run_rows(case, **shape)
     assert torch.equal(before[:270], after[:270]) and after[270:].isnan().all()
+
+
+@pytest.mark.parametrize("heads", [(2, 2, 64), (8, 1, 128)])
+def test_many_single_tokens_give_the_bits_they_give_alone(heads):
+    """More (token, kv head) pairs than one look of the CTAs that deal them out, single tokens and runs in turn."""
+    nq, nkv, d = heads
+    tokens = 40000 // nkv
+    case = paged_case(torch.float32, nq=nq, nkv=nkv, d=d, page=16, lengths=[300, 40, 70, 290], queries=[1, 1, 1, 1], seed=d)
+    g = torch.Generator().manual_seed(nq)
+    rows = torch.arange(tokens, dtype=torch.int32) % 3
+    rows[100:140], rows[1000:1003], rows[tokens - 5:] = 3, 3, 3                # long runs, and one of three
+    limits = torch.tensor([300, 40, 70, 290])[rows.long()]
+    picked = dict(case, token_row=rows.to(DEV), positions=(torch.rand(tokens, generator=g) * limits).int().to(DEV),
+                  q=torch.randn(tokens, nq * d, generator=g).to(DEV))
+    shape = dict(nq=nq, nkv=nkv, d=d, scale=d ** -0.5, window=None)
+    walked = run_rows(picked, **shape, max_chunks=0)
+    for at in (0, 96, 130, 990, tokens // 2, tokens - 60):
+        part = some_rows(picked, slice(at, at + 60))
+        assert torch.equal(run_rows(part, **shape, max_chunks=2), walked[at:at + 60]), at
+
+
+def test_single_tokens_run_side_by_side():
+    """Decoded tokens of many requests, whose chunks are walked: 32 of them take about as long as one (in line they would
+    take 16 times as long)."""
+    times = []
+    for count in (1, 32):
+        case = paged_case(torch.float32, nq=16, nkv=8, d=128, page=16, lengths=[250] * count, queries=[1] * count, seed=count)
+        case = {name: value.to(DEV) if torch.is_tensor(value) else value for name, value in case.items()}
+        call = lambda: run_rows(case, nq=16, nkv=8, d=128, scale=128 ** -0.5, window=None, max_chunks=0)
+        call()
+        best = float("inf")
+        for _ in range(20):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            for _ in range(5):
+                call()
+            end.record()
+            end.synchronize()
+            best = min(best, start.elapsed_time(end))
+        times.append(best)
+    assert times[1] < 5 * times[0], times

@@ -4,27 +4,34 @@
 // A row's keys are cut into chunks of ATTN_CHUNK at absolute multiples, as in the row kernel.  Within a chunk: scores
 // are chains over the dimension; the weights are taken relative to the largest score of the chunk; their sum is 32
 // ascending chains (keys l, l + 32, ...) and a tree over those; an output is the sum of one chain over each 64 keys, in
-// ascending order; chunks are merged in ascending order by merge_partial.  Both kernels below follow that order to
+// ascending order; chunks are merged in ascending order by merge_partial.  All kernels below follow that order to
 // the bit, so a position's result depends neither on the batch nor on how the tokens were cut into steps.
 //
-//  * attention_f32_token_kernel: one CTA a (token, kv head, chunk): decoded tokens.  Bound by reading the keys and
-//    values once; all of a chunk's keys and half its values are in flight at once.
-//  * attention_f32_tile_kernel: one CTA a kv head and 32 query rows (32 / group consecutive tokens with the group's
-//    heads), keys and values in halves of a chunk through two buffers: prompt portions.  Bound by the float32 cores and
-//    shared memory (a thread owns 4 x 4 scores, then 4 x 4 outputs).
+// Tokens are attended in one of two ways:
+//  * F32Token: a CTA a (token, kv head): decoded tokens.  Bound by reading the keys and values once; all of a chunk's keys
+//    and half its values are in flight at once.
+//  * f32_tile: a CTA a kv head and 32 query rows (32 / group consecutive tokens with the group's heads), keys and values in
+//    halves of a chunk through two buffers: runs of four tokens of a request and more within such a tile (prompt portions).
+//    Bound by the float32 cores and shared memory (a thread owns 4 x 4 scores, then 4 x 4 outputs).
+// Mode split has a launch for each, a CTA a chunk.  In mode rows, where a CTA walks all chunks, one launch has both: the first
+// CTAs deal out the tokens outside of runs among themselves, the others have a tile each.  (Tiles that took single tokens
+// in line, each at the cost of 32 rows, needed 358 us for 32 decoded tokens of 200 keys, and 1,547 for 24 of 1,000 keys
+// beside a prompt of 300; these need 16 and 96.)
 //
 // Measured (16 query heads, 8 kv heads of 128, us a layer; one warp a (token, head) that reads every key's row by a lane of
-// its own / these): three prompts of 301, 226 and 151 tokens 403 / 66, one of 600 852 / 120, 100 tokens behind 800
-// beside 100 behind 300 638 / 119; decoding 4 requests of up to 701 tokens 283 / 12, 48 of 701 315 / 82, one of 4,001
-// 292 / 20; a prompt of 9 tokens 8.5 / 12.8 (a tile's fixed cost).
+// its own / these): three prompts of 301, 226 and 151 tokens 373 / 67, one of 600 837 / 119, one of 2,048 8,545 / 840, one
+// of 9 8.5 / 4.5, one of 31 17.9 / 15.7; decoding, mode split: 4 requests of 701 tokens 126 / 13, 48 of 701 309 / 83; mode
+// rows: 4 of 200 98 / 8.3, 32 of 200 100 / 16, 256 of 100 246 / 74, 24 of 1,000 beside a prompt of 300 1,090 / 96.  Prompts of
+// a few tokens each are slower than with a warp a row: 64 of 3 tokens 11 / 31, 32 of 8 15 / 25.
 #pragma once
 
 #define F32_THREADS 256
 #define F32_ROWS 32                        // query rows of a tile
 #define F32_HALF 128                       // keys of a buffer
 #define F32_SUB 64                         // keys of one chain of an output
-#define F32_MIN_RUN 4                      // consecutive tokens of a request from which the tile kernel takes them in mode split
+#define F32_MIN_RUN 4                      // consecutive tokens of a request from which they are attended in a tile
 #define F32_SCORE_ROW (ATTN_CHUNK + 4)
+#define F32_SMS 148                        // one CTA of shared memory this large an SM
 
 struct F32Args {
     const float* q;
@@ -42,14 +49,14 @@ struct F32Args {
     float scale;
 };
 
-// Whether `token` belongs to the tile kernel in mode split: its run of tokens of one request, within the tile of
-// `tile_tokens` it falls into, is long enough.
+// Whether `token` is attended in a tile: its run of tokens of one request, within the tile of `tile_tokens` it
+// falls into, is long enough.
 __device__ __forceinline__ bool f32_in_long_run(const F32Args& a, int token, int tile_tokens) {
     const int from = token - token % tile_tokens, to = min(a.tokens, from + tile_tokens);
     const int request = a.token_row[token];
     int run = 1;
-    for (int t = token - 1; t >= from && a.token_row[t] == request; --t) ++run;
-    for (int t = token + 1; t < to && a.token_row[t] == request; ++t) ++run;
+    for (int t = token - 1; run < F32_MIN_RUN && t >= from && a.token_row[t] == request; --t) ++run;
+    for (int t = token + 1; run < F32_MIN_RUN && t < to && a.token_row[t] == request; ++t) ++run;
     return run >= F32_MIN_RUN;
 }
 
@@ -80,126 +87,205 @@ __device__ __forceinline__ void f32_weights(float* scores, int begin, int lo, in
     sum = warp_sum(sum);
 }
 
+// What a CTA keeps in static shared memory
+struct F32Shared {
+    int64_t slots[ATTN_CHUNK];
+    int row_position[F32_ROWS];                                    // tiles: -1: not a row of this run
+    float row_max[F32_ROWS], row_sum[F32_ROWS];
+};
+
+// One token, one kv head, one chunk: leaves (max, sum) of the group's heads in sh.row_max, sh.row_sum and the sums over 64
+// keys each in `subs`, with a barrier behind.
+template <int D, int GROUP> struct F32Token {
+    static constexpr int PITCH = D + 4;                            // 16 bytes more, for the banks
+    static constexpr int shared_floats = ATTN_CHUNK * PITCH + F32_HALF * D + GROUP * D + GROUP * F32_SCORE_ROW;
+    static_assert(F32_HALF * D + ATTN_CHUNK / F32_SUB * GROUP * D <= ATTN_CHUNK * PITCH, "the sums take the keys' place");
+    float* keys;                                                   // [ATTN_CHUNK][PITCH]; later the values from F32_HALF on
+    float* values;                                                 // [F32_HALF][D]
+    float* q;                                                      // [GROUP][D]
+    float* scores;                                                 // [GROUP][F32_SCORE_ROW]
+    float* subs;                                                   // [ATTN_CHUNK / F32_SUB][GROUP][D], behind the values in keys
+
+    __device__ __forceinline__ explicit F32Token(float* shared) {
+        keys = shared;
+        values = keys + ATTN_CHUNK * PITCH;
+        q = values + F32_HALF * D;
+        scores = q + GROUP * D;
+        subs = keys + F32_HALF * D;
+    }
+
+    __device__ __forceinline__ void load_q(const F32Args& a, int token, int kv_head) {
+        const float* q_rows = a.q + (int64_t)token * a.q_token_stride + (int64_t)kv_head * GROUP * D;
+        for (int i = threadIdx.x; i < GROUP * D; i += F32_THREADS) q[i] = q_rows[i];
+    }
+
+    __device__ __forceinline__ void chunk(const F32Args& a, F32Shared& sh, const int* table, int kv_head, int chunk, int lo,
+                                          int position) {
+        const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+        const int begin = chunk * ATTN_CHUNK;
+        const int first = max(lo, begin) - begin, count = min(position - begin + 1, ATTN_CHUNK);      // keys first..count-1
+        if (tid >= first && tid < count) sh.slots[tid] = f32_slot(a, table, kv_head, begin + tid);
+        __syncthreads();
+        auto load = [&](float* dst, int pitch, const float* cache, int from, int to) {
+            from = max(from, first);
+            to = min(to, count);
+            for (int i = from * (D / 4) + tid; i < to * (D / 4); i += F32_THREADS) {
+                const int j = i / (D / 4), part = i % (D / 4) * 4;
+                cp_async_16(dst + j * pitch + part, cache + sh.slots[j] * D + part, true);
+            }
+            cp_async_commit();
+        };
+        load(keys, PITCH, a.key_cache, 0, ATTN_CHUNK);
+        load(values, D, a.value_cache, 0, F32_HALF);
+        cp_async_wait<1>();
+        __syncthreads();
+        if (tid >= first && tid < count) {
+            float dot[GROUP];
+#pragma unroll
+            for (int g = 0; g < GROUP; ++g) dot[g] = 0.0f;
+            const float4* k4 = reinterpret_cast<const float4*>(keys + tid * PITCH);
+#pragma unroll 8
+            for (int i = 0; i < D / 4; ++i) {
+                const float4 k = k4[i];
+#pragma unroll
+                for (int g = 0; g < GROUP; ++g) {
+                    const float4 v = reinterpret_cast<const float4*>(q + g * D)[i];
+                    dot[g] = __fmaf_rn(v.x, k.x, dot[g]);
+                    dot[g] = __fmaf_rn(v.y, k.y, dot[g]);
+                    dot[g] = __fmaf_rn(v.z, k.z, dot[g]);
+                    dot[g] = __fmaf_rn(v.w, k.w, dot[g]);
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < GROUP; ++g) scores[g * F32_SCORE_ROW + tid] = __fmul_rn(dot[g], a.scale);
+        }
+        __syncthreads();                                           // the keys are read: the other values take their place
+        load(keys - F32_HALF * D, D, a.value_cache, F32_HALF, ATTN_CHUNK);
+        if (warp < GROUP) {
+            float max, sum;
+            f32_weights(scores + warp * F32_SCORE_ROW, begin, lo, position, lane, max, sum);
+            if (lane == 0) { sh.row_max[warp] = max; sh.row_sum[warp] = sum; }
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        const int dim = tid % D;
+        for (int sub = tid / D; sub < ATTN_CHUNK / F32_SUB; sub += F32_THREADS / D) {
+            float acc[GROUP];
+#pragma unroll
+            for (int g = 0; g < GROUP; ++g) acc[g] = 0.0f;
+            const int from = max(sub * F32_SUB, first), to = min((sub + 1) * F32_SUB, count);
+            const float* v = (sub * F32_SUB < F32_HALF ? values : keys - F32_HALF * D) + dim;
+#pragma unroll 8
+            for (int j = from; j < to; ++j) {
+                const float value = v[j * D];
+#pragma unroll
+                for (int g = 0; g < GROUP; ++g) acc[g] = __fmaf_rn(scores[g * F32_SCORE_ROW + j], value, acc[g]);
+            }
+#pragma unroll
+            for (int g = 0; g < GROUP; ++g) subs[(sub * GROUP + g) * D + dim] = acc[g];
+        }
+        __syncthreads();
+    }
+
+    // output i (of GROUP * D) of the chunk
+    __device__ __forceinline__ float output(int i) const {
+        float o = subs[i];
+#pragma unroll
+        for (int sub = 1; sub < ATTN_CHUNK / F32_SUB; ++sub) o = __fadd_rn(o, subs[sub * GROUP * D + i]);
+        return o;
+    }
+};
+
+template <int D, int GROUP>
+__device__ __forceinline__ void f32_zero_token(const F32Args& a, int token, int kv_head) {
+    for (int i = threadIdx.x; i < GROUP * D; i += F32_THREADS)
+        a.out[(int64_t)token * a.out_token_stride + (int64_t)kv_head * GROUP * D + i] = 0.0f;
+}
+
+// Mode split: a CTA a (token, kv head, chunk), partials to scratch; tile_tokens > 0: but for the tokens of long runs.
 template <int D, int GROUP>
 __global__ void __launch_bounds__(F32_THREADS) attention_f32_token_kernel(F32Args a, int tile_tokens) {
-    constexpr int PITCH = D + 4;                                   // 16 bytes more, for the banks
     extern __shared__ __align__(16) float f32_shared[];
-    float* keys = f32_shared;                                      // [ATTN_CHUNK][PITCH]; later the values from F32_HALF on
-    float* values = keys + ATTN_CHUNK * PITCH;                     // [F32_HALF][D]
-    float* q = values + F32_HALF * D;                              // [GROUP][D]
-    float* scores = q + GROUP * D;                                 // [GROUP][F32_SCORE_ROW]
-    float* subs = scores + GROUP * F32_SCORE_ROW;                  // [ATTN_CHUNK / F32_SUB][GROUP][D]
-    __shared__ int64_t slots[ATTN_CHUNK];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int token = blockIdx.x / a.num_kv, kv_head = blockIdx.x % a.num_kv, chunk = blockIdx.y;
+    __shared__ F32Shared sh;
+    const int tid = threadIdx.x, token = blockIdx.x / a.num_kv, kv_head = blockIdx.x % a.num_kv, chunk = blockIdx.y;
     const int position = a.positions[token], request = a.token_row[token];
     if (request < 0 || position < 0) {                             // padding row of a captured batch
-        if (chunk == 0)
-            for (int i = tid; i < GROUP * D; i += F32_THREADS)
-                a.out[(int64_t)token * a.out_token_stride + (int64_t)kv_head * GROUP * D + i] = 0.0f;
+        if (chunk == 0) f32_zero_token<D, GROUP>(a, token, kv_head);
         return;
     }
     const int lo = a.window > 0 ? max(0, position - a.window + 1) : 0;
     if (!chunk_visible(chunk, lo, 0, position)) return;
     if (tile_tokens > 0 && f32_in_long_run(a, token, tile_tokens)) return;
-    const int begin = chunk * ATTN_CHUNK;
-    const int first = max(lo, begin) - begin, count = min(position - begin + 1, ATTN_CHUNK);      // keys first..count-1
-    const int* table = a.block_tables + (int64_t)request * a.table_stride;
-    if (tid >= first && tid < count) slots[tid] = f32_slot(a, table, kv_head, begin + tid);
-    const float* q_rows = a.q + (int64_t)token * a.q_token_stride + (int64_t)kv_head * GROUP * D;
-    for (int i = tid; i < GROUP * D; i += F32_THREADS) q[i] = q_rows[i];
-    __syncthreads();
-    auto load = [&](float* dst, int pitch, const float* cache, int from, int to) {
-        from = max(from, first);
-        to = min(to, count);
-        for (int i = from * (D / 4) + tid; i < to * (D / 4); i += F32_THREADS) {
-            const int j = i / (D / 4), part = i % (D / 4) * 4;
-            cp_async_16(dst + j * pitch + part, cache + slots[j] * D + part, true);
-        }
-        cp_async_commit();
-    };
-    load(keys, PITCH, a.key_cache, 0, ATTN_CHUNK);
-    load(values, D, a.value_cache, 0, F32_HALF);
-    cp_async_wait<1>();
-    __syncthreads();
-    if (tid >= first && tid < count) {
-        float dot[GROUP];
-#pragma unroll
-        for (int g = 0; g < GROUP; ++g) dot[g] = 0.0f;
-        const float4* k4 = reinterpret_cast<const float4*>(keys + tid * PITCH);
-#pragma unroll 8
-        for (int i = 0; i < D / 4; ++i) {
-            const float4 k = k4[i];
-#pragma unroll
-            for (int g = 0; g < GROUP; ++g) {
-                const float4 v = reinterpret_cast<const float4*>(q + g * D)[i];
-                dot[g] = __fmaf_rn(v.x, k.x, dot[g]);
-                dot[g] = __fmaf_rn(v.y, k.y, dot[g]);
-                dot[g] = __fmaf_rn(v.z, k.z, dot[g]);
-                dot[g] = __fmaf_rn(v.w, k.w, dot[g]);
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < GROUP; ++g) scores[g * F32_SCORE_ROW + tid] = __fmul_rn(dot[g], a.scale);
-    }
-    __syncthreads();                                               // the keys are read: the other values take their place
-    load(keys - F32_HALF * D, D, a.value_cache, F32_HALF, ATTN_CHUNK);
+    F32Token<D, GROUP> work(f32_shared);
+    work.load_q(a, token, kv_head);
+    work.chunk(a, sh, a.block_tables + (int64_t)request * a.table_stride, kv_head, chunk, lo, position);
     const int64_t row0 = (int64_t)token * a.num_q + kv_head * GROUP;
-    if (warp < GROUP) {
-        float max, sum;
-        f32_weights(scores + warp * F32_SCORE_ROW, begin, lo, position, lane, max, sum);
-        float* dst = a.scratch + ((row0 + warp) * a.max_chunks + chunk) * (int64_t)(D + 2);
-        if (lane == 0) { dst[0] = max; dst[1] = sum; }
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    const int dim = tid % D;
-    for (int sub = tid / D; sub < ATTN_CHUNK / F32_SUB; sub += F32_THREADS / D) {
-        float acc[GROUP];
-#pragma unroll
-        for (int g = 0; g < GROUP; ++g) acc[g] = 0.0f;
-        const int from = max(sub * F32_SUB, first), to = min((sub + 1) * F32_SUB, count);
-        const float* v = (sub * F32_SUB < F32_HALF ? values : keys - F32_HALF * D) + dim;
-#pragma unroll 8
-        for (int j = from; j < to; ++j) {
-            const float value = v[j * D];
-#pragma unroll
-            for (int g = 0; g < GROUP; ++g) acc[g] = __fmaf_rn(scores[g * F32_SCORE_ROW + j], value, acc[g]);
-        }
-#pragma unroll
-        for (int g = 0; g < GROUP; ++g) subs[(sub * GROUP + g) * D + dim] = acc[g];
-    }
-    __syncthreads();
     for (int i = tid; i < GROUP * D; i += F32_THREADS) {
-        float o = subs[i];
-#pragma unroll
-        for (int sub = 1; sub < ATTN_CHUNK / F32_SUB; ++sub) o = __fadd_rn(o, subs[sub * GROUP * D + i]);
-        a.scratch[((row0 + i / D) * a.max_chunks + chunk) * (int64_t)(D + 2) + 2 + i % D] = o;
+        float* dst = a.scratch + ((row0 + i / D) * a.max_chunks + chunk) * (int64_t)(D + 2);
+        if (i % D == 0) { dst[0] = sh.row_max[i / D]; dst[1] = sh.row_sum[i / D]; }
+        dst[2 + i % D] = work.output(i);
     }
 }
 
-// Mode rows (SPLIT false): every run of tokens of one request, all its chunks.  Mode split: the runs of F32_MIN_RUN
-// tokens and more, chunk blockIdx.y, partials to scratch.
+// Mode rows, one token and kv head: its chunks one after the other, merged as they come.
+template <int D, int GROUP>
+__device__ __forceinline__ void f32_whole_token(const F32Args& a, float* shared, F32Shared& sh, int token, int kv_head) {
+    const int position = a.positions[token], request = a.token_row[token];
+    if (request < 0 || position < 0) {
+        f32_zero_token<D, GROUP>(a, token, kv_head);
+        return;
+    }
+    constexpr int EACH = (GROUP * D + F32_THREADS - 1) / F32_THREADS;      // outputs of a thread
+    const int lo = a.window > 0 ? max(0, position - a.window + 1) : 0;
+    F32Token<D, GROUP> work(shared);
+    Partial<1> total[EACH];
+#pragma unroll
+    for (int e = 0; e < EACH; ++e) total[e] = Partial<1>{-INFINITY, 0.0f, {0.0f}};
+    __syncthreads();                                               // the token before is finished with shared memory
+    work.load_q(a, token, kv_head);
+    for (int chunk = lo / ATTN_CHUNK; chunk <= position / ATTN_CHUNK; ++chunk) {
+        work.chunk(a, sh, a.block_tables + (int64_t)request * a.table_stride, kv_head, chunk, lo, position);
+#pragma unroll
+        for (int e = 0; e < EACH; ++e) {
+            const int i = threadIdx.x + e * F32_THREADS;
+            if (i < GROUP * D) merge_partial(total[e], Partial<1>{sh.row_max[i / D], sh.row_sum[i / D], {work.output(i)}});
+        }
+        __syncthreads();                                           // the sums are read
+    }
+    float* to = a.out + (int64_t)token * a.out_token_stride + (int64_t)kv_head * GROUP * D;
+#pragma unroll
+    for (int e = 0; e < EACH; ++e) {
+        const int i = threadIdx.x + e * F32_THREADS;
+        if (i < GROUP * D) to[i] = __fdiv_rn(total[e].out[0], total[e].sum);
+    }
+}
+
+// A tile's runs of F32_MIN_RUN tokens and more.  SPLIT false: all their chunks; SPLIT: chunk blockIdx.y, partials to scratch.
+template <int D, int GROUP> struct F32Tile {
+    static constexpr int PITCH = D + 4;
+    static constexpr int TOKENS = F32_ROWS / GROUP;
+    static constexpr int shared_floats = 2 * F32_HALF * PITCH + F32_ROWS * PITCH + F32_ROWS * F32_SCORE_ROW;
+};
+
 template <int D, int GROUP, bool SPLIT>
-__global__ void __launch_bounds__(F32_THREADS) attention_f32_tile_kernel(F32Args a) {
-    constexpr int PITCH = D + 4;
-    constexpr int TOKENS = F32_ROWS / GROUP;
+__device__ __forceinline__ void f32_tile(const F32Args& a, float* shared, F32Shared& sh, int block) {
+    constexpr int PITCH = F32Tile<D, GROUP>::PITCH, TOKENS = F32Tile<D, GROUP>::TOKENS;
     constexpr int RT = D / 32;                                     // rows of a thread's outputs (times 4 dims)
     constexpr int DIM_GROUPS = D / 4, ROW_GROUPS = F32_THREADS / DIM_GROUPS;
-    extern __shared__ __align__(16) float f32_shared[];
-    float* buffer[2] = {f32_shared, f32_shared + F32_HALF * PITCH};        // [F32_HALF][PITCH] each
-    float* q = f32_shared + 2 * F32_HALF * PITCH;                  // [F32_ROWS][PITCH]
+    float* buffer[2] = {shared, shared + F32_HALF * PITCH};        // [F32_HALF][PITCH] each
+    float* q = shared + 2 * F32_HALF * PITCH;                      // [F32_ROWS][PITCH]
     float* scores = q + F32_ROWS * PITCH;                          // [F32_ROWS][F32_SCORE_ROW]
-    __shared__ int64_t slots[ATTN_CHUNK];
-    __shared__ int row_position[F32_ROWS];                         // -1: not a row of this run
-    __shared__ float row_max[F32_ROWS], row_sum[F32_ROWS];
+    int64_t* slots = sh.slots;
+    int* row_position = sh.row_position;
+    float* row_max = sh.row_max;
+    float* row_sum = sh.row_sum;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int kv_head = blockIdx.x % a.num_kv, first_token = blockIdx.x / a.num_kv * TOKENS;
+    const int kv_head = block % a.num_kv, first_token = block / a.num_kv * TOKENS;
     const int tile_end = min(a.tokens, first_token + TOKENS);
     const int score_row = (warp & 1) * 4 + (lane & 3), score_key = (warp >> 1) * 8 + (lane >> 2);      // + 8 i, + 32 j
     const int out_row = tid / DIM_GROUPS, out_dim = tid % DIM_GROUPS * 4;                               // + ROW_GROUPS i
 
-    int taken_to = first_token;                                    // mode split: the end of the last run that is this kernel's
+    int taken_to = first_token;                                    // the end of the last run that is taken here
     for (int run = first_token, run_end; run < tile_end; run = run_end) {
         const int request = a.token_row[run];
         int largest = a.positions[run], smallest = largest;
@@ -207,8 +293,8 @@ __global__ void __launch_bounds__(F32_THREADS) attention_f32_tile_kernel(F32Args
             largest = max(largest, a.positions[run_end]);
             smallest = min(smallest, a.positions[run_end]);
         }
-        if (SPLIT && run_end > taken_to) {                         // (equal: the rest of a run that was cut below)
-            if (run_end - run < F32_MIN_RUN) continue;             // the token kernel's
+        if (run_end > taken_to) {                                  // (equal: the rest of a run that was cut below)
+            if (run_end - run < F32_MIN_RUN) continue;             // its tokens are attended one by one
             taken_to = run_end;
         }
         if (request < 0 || smallest < 0) {
@@ -406,29 +492,67 @@ __global__ void __launch_bounds__(F32_THREADS) attention_f32_tile_kernel(F32Args
 }
 
 template <int D, int GROUP>
+__global__ void __launch_bounds__(F32_THREADS, D == 64 ? 2 : 1) attention_f32_tile_kernel(F32Args a) {
+    extern __shared__ __align__(16) float f32_shared[];
+    __shared__ F32Shared sh;
+    f32_tile<D, GROUP, true>(a, f32_shared, sh, blockIdx.x);
+}
+
+// Mode rows.  The first `token_ctas` CTAs deal out the tokens outside of long runs (tile_tokens == 0: all tokens) by kv
+// head, the others have a tile each.  A thread looks at one (token, kv head) of its CTA's share at a time.
+template <int D, int GROUP>
+__global__ void __launch_bounds__(F32_THREADS, D == 64 ? 2 : 1) attention_f32_rows_kernel(F32Args a, int token_ctas, int tile_tokens) {
+    extern __shared__ __align__(16) float f32_shared[];
+    __shared__ F32Shared sh;
+    __shared__ uint32_t taken[F32_THREADS / 32];
+    if ((int)blockIdx.x >= token_ctas) {
+        f32_tile<D, GROUP, false>(a, f32_shared, sh, blockIdx.x - token_ctas);
+        return;
+    }
+    const int items = a.tokens * a.num_kv;
+    for (int64_t base = blockIdx.x; base < items; base += (int64_t)token_ctas * F32_THREADS) {
+        const int64_t at = base + (int64_t)token_ctas * threadIdx.x;
+        const bool mine = at < items && (tile_tokens == 0 || !f32_in_long_run(a, (int)at / a.num_kv, tile_tokens));
+        const uint32_t bits = __ballot_sync(0xffffffffu, mine);
+        __syncthreads();                                           // the share before is read
+        if (threadIdx.x % 32 == 0) taken[threadIdx.x / 32] = bits;
+        __syncthreads();
+        for (int w = 0; w < F32_THREADS / 32; ++w)
+            for (uint32_t left = taken[w]; left; left &= left - 1) {
+                const int item = (int)(base + (int64_t)token_ctas * (w * 32 + __ffs(left) - 1));
+                f32_whole_token<D, GROUP>(a, f32_shared, sh, item / a.num_kv, item % a.num_kv);
+            }
+    }
+}
+
+template <int D, int GROUP>
 static int launch_f32(const F32Args& a, cudaStream_t s) {
-    constexpr int PITCH = D + 4, TOKENS = F32_ROWS / GROUP;
-    constexpr int tile_shared = 4 * (2 * F32_HALF * PITCH + F32_ROWS * PITCH + F32_ROWS * F32_SCORE_ROW);
-    constexpr int token_shared = 4 * (ATTN_CHUNK * PITCH + F32_HALF * D + GROUP * D + GROUP * F32_SCORE_ROW +
-                                      ATTN_CHUNK / F32_SUB * GROUP * D);
+    constexpr int TOKENS = F32Tile<D, GROUP>::TOKENS;
+    constexpr int tile_shared = 4 * F32Tile<D, GROUP>::shared_floats, token_shared = 4 * F32Token<D, GROUP>::shared_floats;
+    constexpr int rows_shared = tile_shared > token_shared ? tile_shared : token_shared;
     const long long tiles = (long long)((a.tokens + TOKENS - 1) / TOKENS) * a.num_kv;
-    if (tiles > 2147483647LL || (long long)a.tokens * a.num_kv > 2147483647LL) return TVB_BAD_ARGUMENT;
+    if (tiles > 2147483647LL - F32_SMS || (long long)a.tokens * a.num_kv > 2147483647LL) return TVB_BAD_ARGUMENT;
     cudaError_t e;
+    // Up to TOKENS tokens each gets a CTA (a chunk) of its own; with more, runs of one request share their keys' reads.
     if (a.max_chunks == 0) {
-        auto kernel = attention_f32_tile_kernel<D, GROUP, false>;
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_shared);
+        // ... from as many on as would go to an SM three at a time: two single tokens take an SM about as long as a tile
+        const int items = a.tokens * a.num_kv;
+        const bool tiled = a.tokens > TOKENS && items > 2 * F32_SMS;
+        auto kernel = attention_f32_rows_kernel<D, GROUP>;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_shared);
         if (e != cudaSuccess) return (int)e;
-        kernel<<<(unsigned)tiles, F32_THREADS, tile_shared, s>>>(a);
+        const int token_ctas = tiled ? F32_SMS : items;
+        kernel<<<(unsigned)(token_ctas + (tiled ? tiles : 0)), F32_THREADS, tiled ? rows_shared : token_shared, s>>>(
+            a, token_ctas, tiled ? TOKENS : 0);
         return tvb_last_error();
     }
-    // Up to TOKENS tokens each gets a CTA a chunk of its own; with more, runs of one request share their keys' reads.
     const bool tiled = a.tokens > TOKENS;
     auto kernel = attention_f32_token_kernel<D, GROUP>;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, token_shared);
     if (e != cudaSuccess) return (int)e;
     kernel<<<dim3((unsigned)(a.tokens * a.num_kv), a.max_chunks), F32_THREADS, token_shared, s>>>(a, tiled ? TOKENS : 0);
     if (tiled) {
-        auto tile_kernel = attention_f32_tile_kernel<D, GROUP, true>;
+        auto tile_kernel = attention_f32_tile_kernel<D, GROUP>;
         e = cudaFuncSetAttribute(tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_shared);
         if (e != cudaSuccess) return (int)e;
         tile_kernel<<<dim3((unsigned)tiles, a.max_chunks), F32_THREADS, tile_shared, s>>>(a);
