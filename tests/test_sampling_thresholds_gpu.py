@@ -1,5 +1,8 @@
 """Thresholds of top-k and top-p at vocabularies where a CTA's part of the row is ragged, empty or too long for shared memory:
-the tokens against the plain rules, and ties at the k-th score over the parts' boundaries."""
+the tokens against the plain rules, and ties at the k-th score over the parts' boundaries; batches whose greedy rows have a
+launch of their own."""
+
+import functools
 
 import pytest
 import torch
@@ -33,3 +36,52 @@ def test_ties_stay_by_token_id_across_parts(at):
     if (at + 1) % vocab in equals:
         kept = {(at + 1) % vocab} | set([i for i in equals if i != (at + 1) % vocab][:wanted - 1])
     assert seen == kept if len(equals) >= wanted - 1 else kept <= seen
+
+
+VOCAB = 151936
+KINDS = {"greedy": [(0.0, 0, 1.0)], "sampled": [(0.8, 50, 1.0), (0.8, 0, 0.95), (0.7, 40, 0.9), (1.0, 0, 1.0)],
+         "mixed": [(0.0, 0, 1.0), (0.8, 50, 1.0), (0.0, 7, 0.5), (0.8, 0, 0.95)]}
+
+
+@functools.cache
+def many_logits():
+    return torch.randn(75, VOCAB, generator=torch.Generator().manual_seed(75)) * 2.0
+
+
+@functools.cache
+def wanted(row, temperature, top_k, top_p):
+    return plain.sample(many_logits()[row], temperature, top_k, top_p, row, 3)
+
+
+@pytest.mark.parametrize("kind", sorted(KINDS))
+@pytest.mark.parametrize("count", [37, 38, 48, 64, 75])
+def test_larger_batches_follow_the_plain_rules(count, kind):
+    rows = [(*KINDS[kind][i % len(KINDS[kind])], i, 3) for i in range(count)]
+    got = k().sample_rows(many_logits()[:count].to(DEV), pack(rows)).cpu().tolist()
+    assert got == [wanted(i, *row[:3]) for i, row in enumerate(rows)]
+
+
+@pytest.mark.parametrize("kind", sorted(KINDS))
+@pytest.mark.parametrize("count", [37, 64])
+def test_what_follows_the_sampling_sees_its_tokens(count, kind):
+    """A captured step as the decode graphs have it: sampling, then a copy of the tokens.  The copy is compared, with
+    logits that change from replay to replay."""
+    rows = [(*KINDS[kind][i % len(KINDS[kind])], i, 3) for i in range(count)]
+    packed, every = pack(rows), many_logits().to(DEV)
+    logits, tokens = torch.zeros(count, VOCAB, device=DEV), torch.zeros(count, dtype=torch.int32, device=DEV)
+    copy = torch.zeros_like(tokens)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        k().sample_rows(logits, packed, out=tokens)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            k().sample_rows(logits, packed, out=tokens)
+            copy.copy_(tokens)
+        for shift in range(30):
+            logits.copy_(every[:count].roll(shift + 1, 0))
+            graph.replay()
+            seen = copy.clone()
+            assert torch.equal(seen, k().sample_rows(logits, packed)), shift
+            if kind == "greedy":
+                assert torch.equal(seen, logits.argmax(1).int()), shift

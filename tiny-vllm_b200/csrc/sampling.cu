@@ -415,7 +415,12 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int rows, int vocab,   /
         if (WHICH == OTHER_ROWS && !team.joined) pdl_wait();
         sample_row<T, STAGED, WHICH == GREEDY_ROWS>(team, shared, staged, row, logits, row_stride, vocab, packed, capacity, tokens);
     }
-    if (!team.joined) cluster_wait();
+    if (!team.joined) {
+        // A CTA without a row of its own waits too: with nothing but greedy rows this grid would else end, and what follows
+        // it start, while the launch for the greedy ones still writes its tokens.
+        if (WHICH == OTHER_ROWS) pdl_wait();
+        cluster_wait();
+    }
 }
 
 template <typename T>
