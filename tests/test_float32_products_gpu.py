@@ -11,7 +11,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("n,k", [(1, 1), (7, 127), (65, 128), (130, 516), (1024, 3072), (520, 1024), (4736, 260), (5003, 2044),
-                                 (24, 25600)])
+                                 (24, 25600), (5003, 5632)])
 def test_every_form_gives_a_row_the_same_bits(n, k):
     generator = torch.Generator(device=DEV).manual_seed(n + k)
     a = torch.randn(331, k, generator=generator, device=DEV)

@@ -355,21 +355,46 @@ static bool takes_few(int m, int n, int k) {
     return m <= FEW_ROWS && few_shared_bytes(few_template_rows(m), few_columns(n), 2, k) <= SHARED_LIMIT;
 }
 
-struct TilePlan { int bm, groups_per, splits, groups; };         // rows of a tile, groups a CTA, CTAs a tile, groups in all
+// How a product runs in tiles: rows of a tile, groups a CTA, CTAs a tile, groups in all, columns of c a launch.
+struct TilePlan { int bm, groups_per, splits, groups, cols; };
 
+#define SCRATCH_FLOATS (16LL << 20)                  // the most that partial sums take
+
+// Time (us) of one group of k in `ctas` tiles spread over the SMs: the busiest SM runs three CTAs side by side, then what
+// is left.  Measured for one, two and three CTAs an SM (4,096 x 12,288 and 1,024 x 2,048 at 12 to 2,048 rows).
+// `even`: many short CTAs, whose rounds run into one another: the mean of that and of an even spread.
+static double group_us(long long ctas, int bm, bool even) {
+    static const double together[3][3] = {{11.5, 14.5, 19.0}, {13.0, 20.0, 28.0}, {28.0, 40.0, 50.0}};
+    const double* us = together[bm == 16 ? 0 : bm == 32 ? 1 : 2];
+    const long long most = (ctas + SMS - 1) / SMS;
+    const double rounds = (double)(most / 3) * us[2] + (most % 3 ? us[most % 3 - 1] : 0.0);
+    return most <= 3 || !even ? rounds : 0.5 * (rounds + (double)ctas / (3 * SMS) * us[2]);
+}
+
+// k is cut over the grid where that is quicker by these times, with 3 us a launch more for adding up the partial sums and
+// what writing and reading them takes (6 TB/s).  They take up to 64 MiB: a product whose sums would take more runs a
+// range of columns at a time.  The order of a sum is the same in all plans.
+// Measured (us, whole / cut): 64 x 6,144 x 1,024 58 / 43, 300 x 1,024 x 2,048 111 / 59, 677 x 6,144 x 1,024 269 / 260,
+// 300 x 4,096 x 12,288 1,299 / 902 in two ranges; not cut: 2,048 x 6,144 x 1,024 690 / 739, 1,024 x 4,096 x 1,024 243 / 246.
 static TilePlan tile_plan(int m, int n, int k) {
     TilePlan plan;
     plan.bm = m <= 16 ? 16 : m <= 32 ? 32 : 64;
     plan.groups = plan.groups_per = (k + GROUP - 1) / GROUP;
-    const long long tiles = (long long)((n + BN - 1) / BN) * ((m + plan.bm - 1) / plan.bm);
-    // Time in groups of one tile on one SM: the busiest SM's share, and for partial sums what writing and adding them
-    // costs (300 x 1024 x 2048: 95 us whole, 58 us in four).
-    double best = 0.0;
-    for (int per = plan.groups; per >= 1; --per) {
-        const int splits = (plan.groups + per - 1) / per;
-        if (splits > 65535) break;
-        const double cost = (double)((tiles * splits + SMS - 1) / SMS) * per + (splits > 1 ? 0.5 : 0.0);
-        if (per == plan.groups || cost < best) { best = cost; plan.groups_per = per; }
+    plan.cols = n;
+    const long long tile_rows = (m + plan.bm - 1) / plan.bm;
+    const double whole = plan.groups * group_us((n + BN - 1) / BN * tile_rows, plan.bm, false);
+    const long long fit = SCRATCH_FLOATS / ((long long)plan.groups * m) / BN * BN;      // columns that the scratch holds
+    if (fit > 0) {
+        const long long ranges = (n + fit - 1) / fit;
+        const int cols = (int)(((n + ranges - 1) / ranges + BN - 1) / BN) * BN;
+        double best = 0.985 * whole;
+        for (int per = plan.groups - 1; per >= 1; --per) {
+            const int splits = (plan.groups + per - 1) / per;
+            if (splits > 65535) break;
+            const double cost = (double)((n + cols - 1) / cols) * (per * group_us(cols / BN * tile_rows * splits, plan.bm, true) + 3.0) +
+                                8.0 * plan.groups * m * n / 6e6;
+            if (cost < best) { best = cost; plan.groups_per = per; plan.cols = std::min(n, cols); }
+        }
     }
     plan.splits = (plan.groups + plan.groups_per - 1) / plan.groups_per;
     return plan;
@@ -405,16 +430,19 @@ static int launch_tiles(const float* a, long long lda, const float* w, long long
     constexpr int shared = TILE_STAGES * (BM + BN) * TILE_ROW * 4;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
     if (e != cudaSuccess) return (int)e;
-    const dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM, plan.splits);
-    if (grid.y > 65535) return TVB_BAD_ARGUMENT;
-    kernel<<<grid, (BM / TM) * (BN / TN), shared, s>>>(a, lda, w, ldw, c, ldc, plan.splits > 1 ? partial : nullptr,
-                                                       plan.groups_per, m, n, k);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
-    if (plan.splits > 1) {
-        const long long size = (long long)m * n;
-        const int blocks = (int)std::min<long long>((size + 255) / 256, 8 * SMS);
-        gemm_f32_fold_kernel<<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n);
+    for (int at = 0; at < n; at += plan.cols) {
+        const int cols = std::min(plan.cols, n - at);
+        const dim3 grid((cols + BN - 1) / BN, (m + BM - 1) / BM, plan.splits);
+        if (grid.y > 65535) return TVB_BAD_ARGUMENT;
+        kernel<<<grid, (BM / TM) * (BN / TN), shared, s>>>(a, lda, w + at * ldw, ldw, c + at, ldc,
+                                                           plan.splits > 1 ? partial : nullptr, plan.groups_per, m, cols, k);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return (int)e;
+        if (plan.splits > 1) {
+            const long long size = (long long)m * cols;
+            const int blocks = (int)std::min<long long>((size + 255) / 256, 8 * SMS);
+            gemm_f32_fold_kernel<<<blocks, 256, 0, s>>>(partial, plan.groups, c + at, ldc, m, cols);
+        }
     }
     return tvb_last_error();
 }
@@ -441,7 +469,15 @@ static int gemm_f32(const float* a, long long lda, const float* w, long long ldw
 extern "C" long long tvb_gemm_f32_scratch_floats(int m, int n, int k) {
     if (m <= 0 || n <= 0 || k <= 0 || takes_few(m, n, k)) return 0;
     const TilePlan plan = tile_plan(m, n, k);
-    return plan.splits > 1 ? (long long)plan.groups * m * n : 0;
+    return plan.splits > 1 ? (long long)plan.groups * m * plan.cols : 0;
+}
+
+// kernels that a product of float32 operands launches
+extern "C" int tvb_gemm_f32_launches(int m, int n, int k) {
+    if (m <= 0 || n <= 0 || k <= 0) return 0;
+    if (takes_few(m, n, k)) return 1;
+    const TilePlan plan = tile_plan(m, n, k);
+    return (n + plan.cols - 1) / plan.cols * (plan.splits > 1 ? 2 : 1);
 }
 
 // in_dtype: type of A and W; out_dtype: type of C (float32 output from bfloat16

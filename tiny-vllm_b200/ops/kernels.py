@@ -1864,15 +1864,21 @@ def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = No
     fn = _fn("gemm_simt", "tvb_gemm_nt_simt",
              [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int,
               c_int, c_int, c_void_p, c_void_p])
-    scratch = None
+    scratch, launches = None, 1
     if a.dtype == torch.float32:
-        floats = _fn("gemm_simt", "tvb_gemm_f32_scratch_floats", [c_int, c_int, c_int], c_longlong)(m, n, k)
+        floats = gemm_f32_scratch_floats(m, n, k)
         if floats > 0:           # partial sums of the pieces that k is cut into
             scratch = torch.empty(floats, dtype=torch.float32, device=a.device)
+            launches = _fn("gemm_simt", "tvb_gemm_f32_launches", [c_int, c_int, c_int])(m, n, k)
     _check(fn(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0),
               m, n, k, dtype_tag(a.dtype), dtype_tag(out.dtype), None if scratch is None else scratch.data_ptr(),
-              _stream()), "gemm_nt_simt", 1 if scratch is None else 2)
+              _stream()), "gemm_nt_simt", launches)
     return out
+
+
+def gemm_f32_scratch_floats(m: int, n: int, k: int) -> int:
+    """float32 of scratch that a product of float32 operands takes for partial sums: 64 MiB at most."""
+    return _fn("gemm_simt", "tvb_gemm_f32_scratch_floats", [c_int, c_int, c_int], c_longlong)(m, n, k)
 
 
 # ------------------------------------------------------------------- sampling
