@@ -405,7 +405,8 @@ static int launch_few(const float* a, long long lda, const float* w, long long l
                       int k, cudaStream_t s) {
     auto kernel = gemm_f32_few_kernel<ROWS, COLS, STAGES, ALIGNED>;
     const int shared = (int)few_shared_bytes(ROWS, COLS, STAGES, k);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
+    // (one limit for all k: a smaller one could come between another thread's limit and its launch)
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_LIMIT);
     if (e != cudaSuccess) return (int)e;
     const int resident = std::max(1, SHARED_LIMIT / (shared + 1024));
     const int tiles = (n + COLS - 1) / COLS;

@@ -386,6 +386,7 @@ __global__ void __launch_bounds__(RET_THREADS) retention_scan_kernel(
 // took 122 us for 3,378 tokens of 16 heads of 128, so 78.
 #define CORRECT_COLS 64
 #define CORRECT_TOKENS 64
+#define CORRECT_SHARED(dim) (((dim) * CORRECT_COLS + CORRECT_TOKENS * ((dim) + 4)) * 4)
 __global__ void __launch_bounds__(128) retention_correct_kernel(
     const float* __restrict__ q, const float* __restrict__ parts, const float* __restrict__ decay,
     const int* __restrict__ row_starts, const int* __restrict__ token_row, float* __restrict__ out, int segment, int rows,
@@ -963,8 +964,10 @@ extern "C" int tvb_retention_scan(const float* q, const float* k, const void* v,
                 state, parts, decay, piece_gates, row_starts, state_slots, token_row, segment, heads, per, vdim);
         const float* queries = RET_GATED ? scaled_q : q;
         if (dim % 4 == 0 && vdim % 4 == 0 && (((uintptr_t)queries | (uintptr_t)parts | (uintptr_t)out) & 15) == 0) {
-            const int shared = (dim * CORRECT_COLS + CORRECT_TOKENS * (dim + 4)) * 4;
-            const cudaError_t e = cudaFuncSetAttribute(retention_correct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
+            const int shared = CORRECT_SHARED(dim);
+            // (one limit for all sizes: a smaller one could come between another thread's limit and its launch)
+            const cudaError_t e = cudaFuncSetAttribute(retention_correct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       CORRECT_SHARED(256));
             if (e != cudaSuccess) return (int)e;
             retention_correct_kernel<<<dim3(pieces, heads, (vdim + CORRECT_COLS - 1) / CORRECT_COLS), 128, shared, s>>>(
                 queries, parts, decay, row_starts, token_row, out, segment, rows, heads, dim, vdim);

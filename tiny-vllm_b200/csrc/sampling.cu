@@ -430,7 +430,8 @@ static cudaError_t launch_sample_rows(const void* logits, long long row_stride, 
     const bool staged = part * 4 <= SAMPLE_STAGED_BYTES;
     const int bytes = staged ? (int)part * 4 : 0;
     auto launch = [&](auto kernel, int clusters, int shared) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
+        // (one limit for all sizes: a smaller one could come between another thread's limit and its launch)
+        cudaError_t e = shared ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_STAGED_BYTES) : cudaSuccess;
         if (e != cudaSuccess) return e;
         TvbLaunch launch(dim3(clusters * SAMPLE_CTAS), dim3(SAMPLE_THREADS), shared, s, pdl, SAMPLE_CTAS);
         return cudaLaunchKernelEx(&launch.config, kernel, (const T*)logits, (int64_t)row_stride, rows, vocab, packed, capacity, tokens);
