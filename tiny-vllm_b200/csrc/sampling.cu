@@ -423,13 +423,20 @@ sample_rows_kernel(const T* logits, int64_t row_stride, int rows, int vocab,   /
     }
 }
 
+// bytes of shared memory that a CTA's part of a row takes; 0: more than there is
+static int staged_bytes(int vocab) {
+    const long long part = (((long long)vocab + SAMPLE_CTAS - 1) / SAMPLE_CTAS + 3) / 4 * 4;
+    return part * 4 <= SAMPLE_STAGED_BYTES ? (int)part * 4 : 0;
+}
+
+static bool two_launches(int rows, int vocab) { return rows > SAMPLE_ROWS_AT_ONCE && staged_bytes(vocab) > 0; }
+
+// pdl: 1 for the programmatic launch behind the kernel before, 2 for that of the second launch behind the first
 template <typename T>
 static cudaError_t launch_sample_rows(const void* logits, long long row_stride, int rows, int vocab, const int* packed,
                                       int capacity, int* tokens, int pdl, cudaStream_t s) {
-    const long long part = (((long long)vocab + SAMPLE_CTAS - 1) / SAMPLE_CTAS + 3) / 4 * 4;
-    const bool staged = part * 4 <= SAMPLE_STAGED_BYTES;
-    const int bytes = staged ? (int)part * 4 : 0;
-    auto launch = [&](auto kernel, int clusters, int shared) -> cudaError_t {
+    const int bytes = staged_bytes(vocab);
+    auto launch = [&](auto kernel, int clusters, int shared, int pdl) -> cudaError_t {
         // (one limit for all sizes: a smaller one could come between another thread's limit and its launch)
         cudaError_t e = shared ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_STAGED_BYTES) : cudaSuccess;
         if (e != cudaSuccess) return e;
@@ -439,13 +446,15 @@ static cudaError_t launch_sample_rows(const void* logits, long long row_stride, 
     // The shared memory leaves room for two CTAs an SM.  Rows beyond those that fit at once would make greedy rows,
     // which do not use it, wait in line: they get a launch without it (64 greedy rows of 151,936 tokens: 17.6 us in one
     // launch).
-    if (rows <= SAMPLE_ROWS_AT_ONCE || !staged)
-        return staged ? launch(sample_rows_kernel<T, true, ALL_ROWS>, rows, bytes)
-                      : launch(sample_rows_kernel<T, false, ALL_ROWS>, rows, bytes);
-    const cudaError_t e = launch(sample_rows_kernel<T, false, GREEDY_ROWS>, rows, 0);
-    pdl = 1;                                 // whatever the first launch was: the second waits for it by itself
-    return e != cudaSuccess ? e : launch(sample_rows_kernel<T, true, OTHER_ROWS>, SAMPLE_ROWS_AT_ONCE, bytes);
+    if (!two_launches(rows, vocab))
+        return bytes ? launch(sample_rows_kernel<T, true, ALL_ROWS>, rows, bytes, pdl & 1)
+                     : launch(sample_rows_kernel<T, false, ALL_ROWS>, rows, 0, pdl & 1);
+    const cudaError_t e = launch(sample_rows_kernel<T, false, GREEDY_ROWS>, rows, 0, pdl & 1);
+    return e != cudaSuccess ? e : launch(sample_rows_kernel<T, true, OTHER_ROWS>, SAMPLE_ROWS_AT_ONCE, bytes, pdl >> 1);
 }
+
+// launches that sampling so many rows takes
+extern "C" int tvb_sample_rows_launches(int rows, int vocab) { return rows <= 0 ? 0 : two_launches(rows, vocab) ? 2 : 1; }
 
 // packed: int32 [7, capacity], field-major: temperature and top_p as float bits, top_k,
 // seed low/high word, draw-counter low/high word; row r reads column r.

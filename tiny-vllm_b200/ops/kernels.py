@@ -42,12 +42,13 @@ _launches = 0
 # Programmatic dependent launch for the kernels that wait for their predecessor themselves
 # (griddepcontrol.wait): they may start, and fetch weights, while the kernel before them ends.
 # TINYVLLM_B200_PDL=0 turns it off; a comma-separated list (gemm,norm,attention,attention_few,prefill,
-# sample) keeps it for those kernels only (attention: the decode attention at every batch size;
+# sample,sample_second) keeps it for those kernels only (attention: the decode attention at every batch size;
 # attention_few: with up to PDL_ATTENTION_ROWS rows and only where the launch runs as CTAs of eight
 # warps that are all on the GPU at once, which find the SMs free: batch 1 to 3 gain 3 to 4 %, batch
 # 4 is level and batch 6 loses 3 %, its clusters waiting for room beside the projection's CTAs; prefill: the prompt's q/k norm, rotation and cache write,
-# and the tcgen05 attention).
-_PDL_DEFAULT = ("gemm", "norm", "attention_few")
+# and the tcgen05 attention; sample_second: the launch for the sampled rows of a large batch behind the one
+# for its greedy rows).
+_PDL_DEFAULT = ("gemm", "norm", "attention_few", "sample_second")
 PDL_ATTENTION_ROWS = 3
 _setting = os.environ.get("TINYVLLM_B200_PDL", "1")
 PDL = frozenset() if _setting == "0" else frozenset(_PDL_DEFAULT if _setting == "1" else _setting.split(","))
@@ -1897,8 +1898,10 @@ def sample_rows(logits: torch.Tensor, packed: torch.Tensor, out: torch.Tensor | 
         out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
     fn = _fn("sampling", "tvb_sample_rows",
              [c_void_p, c_longlong, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p])
+    launches = _fn("sampling", "tvb_sample_rows_launches", [c_int, c_int])(rows, vocab)
     _check(fn(logits.data_ptr(), logits.stride(0), rows, vocab, packed.data_ptr(), packed.shape[1],
-              out.data_ptr(), dtype_tag(logits.dtype), _pdl("sample"), _stream()), "sample_rows")
+              out.data_ptr(), dtype_tag(logits.dtype), _pdl("sample") | _pdl("sample_second") << 1, _stream()),
+           "sample_rows", launches)
     return out
 
 
