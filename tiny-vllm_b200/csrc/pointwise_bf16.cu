@@ -5,46 +5,53 @@
 // :153-211, :274-285; tinyvllm/kernels/kv_store.cu:26-90).
 #include "common.cuh"
 
-// Eight weights from p on, as 16-byte words (p on such a boundary).
-__device__ __forceinline__ void load_weights8(const float* p, float* w) {
-    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-    w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+// Eight weights from p on: 16-byte words, where p lies on such a boundary, or one by one
+__device__ __forceinline__ void load_weights8(const float* p, bool in_words, float* w) {
+    if (in_words) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint4 word = ld_global_16(p + 4 * h);
+            w[4 * h] = __uint_as_float(word.x); w[4 * h + 1] = __uint_as_float(word.y);
+            w[4 * h + 2] = __uint_as_float(word.z); w[4 * h + 3] = __uint_as_float(word.w);
+        }
+    } else
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = ld_global_f32(p + e);
 }
-__device__ __forceinline__ void load_weights8(const bf16* p, float* w) {
-    unpack_bf16x8(*reinterpret_cast<const uint4*>(p), w);
-}
-// ... and at any address
-template <typename W> __device__ __forceinline__ void load_weights8(const W* p, bool in_words, float* w) {
-    if (in_words) load_weights8(p, w);
+__device__ __forceinline__ void load_weights8(const bf16* p, bool in_words, float* w) {
+    if (in_words) unpack_bf16x8(ld_global_16(p), w);
     else
 #pragma unroll
-        for (int e = 0; e < 8; ++e) w[e] = to_float<W>(p[e]);
+        for (int e = 0; e < 8; ++e) w[e] = bf16_bits_to_float(ld_global_u16(p + e));
 }
 
 // -------------------------------------------------------------------- RMSNorm
 // TPR threads share a row (32: one warp, 8 rows a CTA; 64, 128; 256: the whole CTA).  A thread holds up to
-// 4 words of 8 values.  `x` and `residual` come from the kernel before: coherent loads.  The weights do not:
-// they are read before the wait for it, in 16-byte words where they lie on such a boundary (read one by one behind the
-// row's sum, 32 bytes from lane to lane, they made it 5.8 us for 2,048 rows of 1,024 instead of 4.2, and 51 for 8,192 of 4,096 instead of 42).
+// 4 words of 8 values.  `x` and `residual` come from the kernel before: coherent loads.  So may the weights, unless the
+// caller says that they were there long ago (weights_constant): then they are read before the wait.  Either way in 16-byte
+// words where they lie on such a boundary (read one by one behind the row's sum, 32 bytes from lane to lane, they made it
+// 5.9 us for 2,048 rows of 1,024; behind the wait 4.8, before it 4.2; 8,192 rows of 4,096 51 and 42 either way).
 #define NORM_WORDS 4
 
 template <int TPR, typename W>
 __global__ void __launch_bounds__(256)
-rms_norm_bf16_kernel(const bf16* x, const bf16* residual, const W* __restrict__ weight,
+rms_norm_bf16_kernel(const bf16* x, const bf16* residual, const W* weight,
                      bf16* __restrict__ y, bf16* __restrict__ residual_out,
-                     const int* __restrict__ gather, int rows, int width, float eps, int weight_words) {
+                     const int* __restrict__ gather, int rows, int width, float eps, int weight_words, int weights_constant) {
     __shared__ float scratch[32];
     __shared__ float row_parts[8];
     const int rows_per_cta = 256 / TPR;
     const int out_row = blockIdx.x * rows_per_cta + threadIdx.x / TPR;
     const int lane = threadIdx.x % TPR;
     float weights[NORM_WORDS][8];
+    auto load_weights = [&]() {
 #pragma unroll
-    for (int i = 0; i < NORM_WORDS; ++i) {
-        const int at = (lane + i * TPR) * 8;
-        if (at < width) load_weights8<W>(weight + at, weight_words, weights[i]);
-    }
+        for (int i = 0; i < NORM_WORDS; ++i) {
+            const int at = (lane + i * TPR) * 8;
+            if (at < width) load_weights8(weight + at, weight_words, weights[i]);
+        }
+    };
+    if (weights_constant) load_weights();
     pdl_wait();
     pdl_launch_dependents();
     const bool live = out_row < rows;
@@ -65,6 +72,7 @@ rms_norm_bf16_kernel(const bf16* x, const bf16* residual, const W* __restrict__ 
             if (rr) r_words[i] = ld_global_16(rr + at);
         }
     }
+    if (!weights_constant) load_weights();
 #pragma unroll
     for (int i = 0; i < NORM_WORDS; ++i) {
         const int at = (lane + i * TPR) * 8;
@@ -113,7 +121,7 @@ extern "C" int tvb_rms_norm_bf16_supports(int width) { return width > 0 && width
 
 extern "C" int tvb_rms_norm_bf16(const void* x, const void* residual, const void* weight, void* y,
                                  void* residual_out, const int* gather, int rows, int width, float eps,
-                                 int weight_dtype, int pdl, void* stream) {
+                                 int weight_dtype, int weights_constant, int pdl, void* stream) {
     if (rows <= 0) return 0;
     if (!tvb_rms_norm_bf16_supports(width)) return TVB_BAD_ARGUMENT;
     // threads that share a row: the fewer rows, the more, so that the GPU is filled either way
@@ -127,7 +135,7 @@ extern "C" int tvb_rms_norm_bf16(const void* x, const void* residual, const void
 #define NORM_LAUNCH(TPR, WT)                                                                          \
     e = cudaLaunchKernelEx(&launch.config, rms_norm_bf16_kernel<TPR, WT>, (const bf16*)x,             \
                            (const bf16*)residual, (const WT*)weight, (bf16*)y, (bf16*)residual_out,   \
-                           gather, rows, width, eps, (int)(((uintptr_t)weight & 15) == 0))
+                           gather, rows, width, eps, (int)(((uintptr_t)weight & 15) == 0), weights_constant)
 #define NORM_BY_TPR(WT)                                        \
     do {                                                       \
         if (tpr == 32) NORM_LAUNCH(32, WT);                    \

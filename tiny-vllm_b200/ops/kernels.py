@@ -187,12 +187,14 @@ def embed_pairs(table: torch.Tensor, ids: torch.Tensor, *, positions: torch.Tens
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, *, residual: torch.Tensor | None = None,
              rows: torch.Tensor | None = None, out: torch.Tensor | None = None,
-             residual_out: torch.Tensor | None = None, want_residual: bool = True):
+             residual_out: torch.Tensor | None = None, want_residual: bool = True, weight_constant: bool = False):
     """RMSNorm over the last dimension of x [tokens, width].
 
     With ``residual`` the rounded sum x + residual is normalised and returned as
     the second result (the new residual stream).  With ``rows`` (int32) only
     those rows are produced, in that order, and no residual is returned.
+    ``weight_constant``: nothing in flight on the stream writes the weight (a model's, loaded
+    before), so it may be read while the launch before still runs.
     """
     _need_cuda(x, weight, residual, rows)
     if x.dim() != 2 or not x.is_contiguous() or weight.shape != (x.shape[1],):
@@ -215,10 +217,10 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, *, residual: tor
     if x.dtype == torch.bfloat16 and width % 8 == 0 and width <= 8192:     # 16-byte accesses
         fn = _fn("pointwise_bf16", "tvb_rms_norm_bf16",
                  [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
-                  c_int, c_int, c_void_p])
+                  c_int, c_int, c_int, c_void_p])
         _check(fn(x.data_ptr(), _ptr(residual), weight.data_ptr(), out.data_ptr(), _ptr(residual_out),
-                  _ptr(rows), count, width, eps, dtype_tag(weight.dtype), _pdl("norm"), _stream()),
-               "rms_norm")
+                  _ptr(rows), count, width, eps, dtype_tag(weight.dtype), 1 if weight_constant else 0, _pdl("norm"),
+                  _stream()), "rms_norm")
         if residual is not None and rows is None:
             return out, residual_out
         return out

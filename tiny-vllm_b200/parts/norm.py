@@ -17,6 +17,7 @@ from .registry import register_part
 class RMSNorm(Part):
     # y = x * rsqrt(mean(x^2) + eps) * weight: a projection behind it may apply it in its own kernel
     folds_into_product = True
+    # (the weights are a loaded model's: no kernel of a step writes them)
 
     def __init__(self, ctx: BuildContext, *, width: int, eps: float, name: str | None = None) -> None:
         self.width = width
@@ -28,15 +29,15 @@ class RMSNorm(Part):
         return [ParamSpec.single("weight", self.name, (self.width,), role="vector", init="around_one")]
 
     def forward(self, x):
-        return kernels.rms_norm(x, self.weight, self.eps)
+        return kernels.rms_norm(x, self.weight, self.eps, weight_constant=True)
 
     def add(self, x, residual):
         """(norm(x + residual), x + residual)"""
-        return kernels.rms_norm(x, self.weight, self.eps, residual=residual)
+        return kernels.rms_norm(x, self.weight, self.eps, residual=residual, weight_constant=True)
 
     def add_rows(self, x, residual, rows):
         """norm(x + residual) on the rows named by ``rows`` only."""
-        return kernels.rms_norm(x, self.weight, self.eps, residual=residual, rows=rows)
+        return kernels.rms_norm(x, self.weight, self.eps, residual=residual, rows=rows, weight_constant=True)
 
 
 class PendingUpdate:
