@@ -53,3 +53,24 @@ def test_an_entry_is_cut_the_same_beside_any_other(count, start, small_context):
         assert cut_of(0, [count, other], [start, at], small_context) == alone
         assert cut_of(1, [other, count], [at, start], small_context) == alone
         assert cut_of(1, [other, count, other], [at, start, at], small_context) == alone
+
+
+def test_asking_whether_windowed_attention_takes_tiles_loads_no_library(monkeypatch):
+    from types import SimpleNamespace
+
+    from tinyvllm_b200.ops.attention import windowed_takes_tensor_memory_tiles
+
+    def loaded(name):
+        raise AssertionError(f"{name} was loaded")
+
+    monkeypatch.setattr(kernels, "load_library", loaded)
+    monkeypatch.setattr(kernels, "_functions", {})
+    mixer = SimpleNamespace(key_dim=128, value_dim=128, softcap=None, distance_slope_exponent=None, segment=1024, window=None,
+                            distance_table=(32, 1024.0), num_heads=16, num_kv_heads=8)
+    assert windowed_takes_tensor_memory_tiles(mixer, 16)
+    mixer.distance_table = (32, float(kernels.PREFILL_TC_BIAS_ROWS))
+    assert not windowed_takes_tensor_memory_tiles(mixer, 16)
+
+
+def test_the_library_takes_as_long_a_bias_as_it_is_said_to():
+    assert kernels._fn("attention_prefill_tc", "tvb_attention_prefill_tc_bias_rows", [])() == kernels.PREFILL_TC_BIAS_ROWS

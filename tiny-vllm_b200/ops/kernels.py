@@ -2153,15 +2153,13 @@ def attention_prefill_tc(q: torch.Tensor, q_token_stride: int, key_cache: torch.
     return out
 
 
-_prefill_tc_bias_rows: int | None = None
+PREFILL_TC_BIAS_ROWS = 2048            # BIAS_ROWS of attention_prefill_tc.cu
 
 
 def attention_prefill_tc_bias_rows() -> int:
-    """Rows (distances) a learned bias may have in :func:`attention_prefill_tc_extras`."""
-    global _prefill_tc_bias_rows
-    if _prefill_tc_bias_rows is None:
-        _prefill_tc_bias_rows = _fn("attention_prefill_tc", "tvb_attention_prefill_tc_bias_rows", [])()
-    return _prefill_tc_bias_rows
+    """Rows (distances) a learned bias may have in :func:`attention_prefill_tc_extras` (answered here, so that a model
+    that asks when it is built loads no library; the library checks the same)."""
+    return PREFILL_TC_BIAS_ROWS
 
 
 def attention_prefill_tc_extras(q: torch.Tensor, key_cache: torch.Tensor, value_cache: torch.Tensor,
