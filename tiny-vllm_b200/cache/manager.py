@@ -23,7 +23,16 @@ the free list is a stack, which reuses them as early.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from itertools import chain
+
+import numpy as np
+
+
+def portion_slots(table, start: int, count: int, page_size: int) -> np.ndarray:
+    """Cache slots (int32) of the positions start to start + count - 1 of a request with this block table: position p lies
+    in slot p % page_size of its page.  Page by page: token by token a prompt of 2,048 tokens took 0.26 ms."""
+    pages = np.array(table[start // page_size:(start + count - 1) // page_size + 1], dtype=np.int32)
+    slots = (pages[:, None] * page_size + np.arange(page_size, dtype=np.int32)).reshape(-1)
+    return slots[start % page_size:start % page_size + count]
 
 
 class CacheError(RuntimeError):
@@ -287,13 +296,10 @@ class CacheManager:
                         raise CacheError("a token would be written to a page already given back")
                     row = (table[p // size] * size + p % size,)
                 else:
-                    # page by page, not token by token: a prompt of 2,048 tokens took 0.26 ms a group
                     first = request.length
-                    touched = table[first // size:(first + count - 1) // size + 1]
-                    if min(touched) < 0:
+                    if min(table[first // size:(first + count - 1) // size + 1]) < 0:
                         raise CacheError("a token would be written to a page already given back")
-                    whole = list(chain.from_iterable(range(page * size, page * size + size) for page in touched))
-                    row = tuple(whole[first % size:first % size + count])
+                    row = tuple(portion_slots(table, first, count, size).tolist())
                 slots.append(row)
                 tables.append(table)
             request.planned = True

@@ -23,7 +23,7 @@ from typing import Sequence
 import numpy as np
 import torch
 
-from ..cache.manager import CacheManager, StepCachePlan
+from ..cache.manager import CacheManager, StepCachePlan, portion_slots
 from ..cache.storage import CacheStorage, bytes_per_page, group_runs
 from ..ops import attention as attention_ops
 from ..ops import kernels
@@ -265,11 +265,8 @@ class StepRunner:
                 table = planned.tables[g]
                 if n == 1:
                     view(6 + 2 * g)[cursor] = planned.slots[g][0]
-                else:                          # planned.slots[g], from the pages instead of token by token
-                    size, at = self.manager.page_size, planned.start
-                    pages = np.array(table[at // size:(at + n - 1) // size + 1], dtype=np.int32)
-                    slots = (pages[:, None] * size + np.arange(size, dtype=np.int32)).reshape(-1)
-                    view(6 + 2 * g)[cursor:cursor + n] = slots[at % size:at % size + n]
+                else:                          # planned.slots[g] by the same rule, without a list of them
+                    view(6 + 2 * g)[cursor:cursor + n] = portion_slots(table, planned.start, n, self.manager.page_size)
                 view(7 + 2 * g)[r * blocks[g]:r * blocks[g] + len(table)] = table
             max_position = max(max_position, planned.start + n - 1)
             cursor += n
