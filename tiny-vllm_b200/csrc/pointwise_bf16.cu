@@ -327,7 +327,8 @@ extern "C" int tvb_qk_norm_rope_store_bf16(void* qkv, const void* q_weight, cons
         return TVB_BAD_ARGUMENT;
     if (head_dim % 8 || ((num_q + 2 * num_kv) * head_dim) % 8) return TVB_BAD_ARGUMENT;
     // a warp per token, eight to a block; from 1,024 tokens on two, so that the last blocks even out over the SMs
-    // (16 q / 8 kv heads, 4,000 tokens 13.9 us with eight, 13.2 with two; 32 / 8, 8,192 tokens 44.3 and 42.3)
+    // (us with eight / two, 16 q / 8 kv heads: 1,024 tokens 6.1 / 6.0, 1,500 7.7 / 6.8, 2,048 7.8 / 7.7, 4,000 13.9 / 13.3,
+    // 8,192 31.0 / 29.4; 32 / 8: 1,024 7.9 / 7.9, 1,500 10.5 / 8.9, 8,192 44.7 / 42.7; below, a block an SM has room either way)
     const int together = tokens >= 1024 ? 2 : 8;
     const int64_t blocks = ((int64_t)tokens + together - 1) / together;
     cudaStream_t s = (cudaStream_t)stream;

@@ -22,8 +22,9 @@
 // one of the cluster.  Rows too long for that (more than about 430,000 tokens) read the logits in every pass.
 //
 // Bound by the passes' barriers and compares.  Measured over 151,936 tokens (us; one bit a pass over the logits in L2 /
-// this): 48 rows, half of them greedy, a quarter top-k 50, a quarter top-p 0.95 684 / 137; one row of top-k 50 499 / 53,
-// of top-p 0.95 647 / 77, of both 1,016 / 91; 64 rows of both 1,096 / 352; one greedy row 4.1 / 4.3, 64 10.6 / 12.5.
+// this): 48 rows, half of them greedy, a quarter top-k 50, a quarter top-p 0.95 680 / 128; one row of top-k 50 496 / 52,
+// of top-p 0.95 645 / 77, of both 1,013 / 89; 64 rows of both 1,083 / 343.  Greedy rows alone are slower for it: one
+// 4.1 / 4.4, 32 4.9 / 5.9, 37 5.1 / 9.6 (33 clusters of this shared memory fit at once), 38 5.1 / 7.5, 64 6.1 / 8.8.
 #include "common.cuh"
 
 #include <cstdint>
@@ -445,7 +446,8 @@ static cudaError_t launch_sample_rows(const void* logits, long long row_stride, 
     };
     // The shared memory leaves room for two CTAs an SM.  Rows beyond those that fit at once would make greedy rows,
     // which do not use it, wait in line: they get a launch without it (64 greedy rows of 151,936 tokens: 17.6 us in one
-    // launch).
+    // launch, 8.8 in two).  With the line at the 33 clusters that fit, 34 to 44 rows were up to 15 % quicker with one kind
+    // of sampling, but mixed rows 9 % slower and 48 rows up to 6 %.
     if (!two_launches(rows, vocab))
         return bytes ? launch(sample_rows_kernel<T, true, ALL_ROWS>, rows, bytes, pdl & 1)
                      : launch(sample_rows_kernel<T, false, ALL_ROWS>, rows, 0, pdl & 1);

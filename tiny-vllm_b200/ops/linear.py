@@ -1,6 +1,6 @@
 """x . W^T for the parts, by storage dtype.
 
-float32: the package's own float32-core kernel (true 32-bit, ascending k).
+float32: the package's own float32-core kernels (true 32-bit; the order of a sum depends on k alone).
 bfloat16: the tensor-core kernels of this package where they take the shape,
 else cuBLAS through ``torch.nn.functional.linear``, which is what the
 reference's engine calls for every projection (tinyvllm/layers.py:84-85).
