@@ -1,0 +1,429 @@
+// C[m, n] = A[m, k] . W[n, k]^T of float32 operands with more than a few rows, on the fifth-generation tensor cores
+// and with the precision of float32 sums.  (Few rows, and rows off the 16-byte boundary: gemm_simt.cu.)
+//
+// A float32 is the sum of three bfloat16, exactly: x1 is x rounded to 8 bits (so that the rest has either sign), x2 the
+// first 8 bits of the rest and x3 what is left.  A product of two such sums is nine products, of which the six largest
+// are taken (x1 w1; x1 w2, x2 w1; x2 w2, x1 w3, x3 w1): what is left out is about 2^-26 of |x w|, with either sign.
+// Products of bfloat16 are exact in float32; the tensor cores add them up in tensor memory over 64 k, the small ones
+// first, and every such sum is then added by the float32 cores to a sum in registers, in ascending order of k: the
+// tensor cores cut off what does not fit instead of rounding it, which over all of k would shrink the sums.
+//
+// The sum of an output element has one order whatever m is: blocks of 64 k ascending inside a group of 1,024, the groups
+// ascending.  Operands with infinities, NaN or values that round to infinity in bfloat16 have no such three parts: the
+// rows and columns that hold one are summed again by the float32 cores from the operands themselves.
+//
+// x is split once, by a small kernel; w on its way into shared memory, by the 16 warps that also add up the sums: its
+// parts are never in memory, and a weight takes no more room than before.  Integer instructions split (the conversion
+// to bfloat16 has a quarter of their rate).  A tile is 128 columns of c by 16 to 128 rows: with two stages of 96 KB no
+// more fits.  A block of 64 k takes 1.4 us at 16 rows and 1.9 at 128, of which the products are 0.6 and 0.9: what bounds
+// the kernel is the chain of splitting, handing over, products and sums, two blocks deep, and shared memory, which the
+// products read at nearly its rate.  (Registers decide: at 96 a thread nothing may spill, since 28 KB of L1 are left and
+// the stream of w evicts what is spilled: 2.2 us a block.  Eight warps that split beside eight that add up: 2.0.)
+//
+// Measured (us, float32 cores / this, weights from memory): 64 rows 4,096 x 1,024 31 / 29, 6,144 x 1,024 43 / 29, 1,024 x
+// 3,072 30 / 31; 301 rows 93 / 33, 127 / 36, 76 / 36; 677 rows 176 / 63, 260 / 70 (121 TFLOP/s), 139 / 46; 2,048 rows
+// 464 / 139, 687 / 196 (132 TFLOP/s), 354 / 122.  Error against 64-bit sums (2-norm) at k = 1,024 / 3,072 / 25,600: 1.10e-7,
+// 1.16e-7, 1.46e-7 (float32 cores 1.55e-7, 1.60e-7, 2.02e-7); of that 6e-8 is what the tensor cores cut off.
+#include <algorithm>
+
+#include "tc5.cuh"
+
+namespace {
+
+constexpr int BW = 128;                 // rows of w of a tile = lanes of tensor memory
+constexpr int MAX_X = 128;              // rows of x of a tile at most; a launch takes a multiple of 16
+constexpr int BK = 64;                  // k of a stage: 64 bfloat16 = 128 bytes = one swizzle row
+constexpr int UMMA_K = 16;
+constexpr int GROUP = 1024;             // k of a sum in registers
+constexpr int GROUP_BLOCKS = GROUP / BK;
+constexpr int WORK_WARPS = 16;          // split w and add up sums; one more warp copies x and issues the products
+constexpr int WORKERS = 32 * WORK_WARPS;
+constexpr int THREADS = WORKERS + 32;
+constexpr int SUM_COLS = MAX_X / (WORK_WARPS / 4);       // rows of x whose sums a warp holds
+constexpr int STAGES = 2;
+constexpr int PART_BYTES = 128 * BK * 2;                 // one of the three parts of 128 rows
+constexpr int STAGE_BYTES = 6 * PART_BYTES;              // of w, then of x
+constexpr int BARRIERS = 4;
+constexpr int SHARED_BYTES = STAGES * STAGE_BYTES + BARRIERS * 8 + 16 + 256 + 1024;
+constexpr uint32_t TMEM_COLS = 2 * MAX_X;
+constexpr int ROWS_A_PASS = WORKERS / (BK / 4);          // 32: a thread takes 4 k of every 32nd row of w
+constexpr int PASSES = 128 / ROWS_A_PASS;
+
+enum { GAVE_UP_FULL = 1, GAVE_UP_DONE = 2, GAVE_UP_FREE = 3 };
+
+__device__ int tvb_gemm_f32_tc_status_word = 0;
+
+// a * b + c on two float32 at once.
+__device__ __forceinline__ float2 fma_two(float2 a, float2 b, float2 c) {
+    union Pair { float2 f; unsigned long long u; } x{a}, y{b}, z{c}, r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.u) : "l"(x.u), "l"(y.u), "l"(z.u));
+    return r.f;
+}
+
+// Four float32 as three times four bfloat16.  `wild` becomes NaN if a value has no such parts.
+__device__ __forceinline__ void split_four(const float4& x, uint2* part, float2& wild) {
+    float2 rest[2] = {make_float2(x.x, x.y), make_float2(x.z, x.w)};
+    uint32_t* words = reinterpret_cast<uint32_t*>(part);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            const uint32_t half = p == 0 ? 0x8000u : 0u;
+            const uint32_t a = __float_as_uint(rest[j].x) + half, b = __float_as_uint(rest[j].y) + half;
+            words[2 * p + j] = __byte_perm(a, b, 0x7632);
+            if (p == 2) break;
+            rest[j] = fma_two(make_float2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)),
+                              make_float2(-1.0f, -1.0f), rest[j]);           // exact
+        }
+        wild = fma_two(rest[j], make_float2(0.0f, 0.0f), wild);
+    }
+}
+
+// One lane of the warp, chosen so that the compiler keeps the control flow of the warp uniform.
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t elected;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.b32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(elected));
+    return elected != 0;
+}
+
+// The sum over [k_from, k_to) by the float32 cores, for operands that cannot be split.
+__device__ float plain_sum(const float* x, const float* w, int k_from, int k_to) {
+    float sum = 0.0f;
+    for (int at = k_from; at < k_to; ++at) sum = __fmaf_rn(x[at], w[at], sum);
+    return sum;
+}
+
+// A row of x a block: its three parts, [3][m][kp] with zeros from k on, and whether it holds a value that has none.
+__global__ void __launch_bounds__(128)
+split_rows_kernel(const float* __restrict__ a, int64_t lda, uint2* parts, int* wild_x, int m, int k, int kp) {
+    pdl_launch_dependents();
+    const int row = blockIdx.x;
+    float2 wild = make_float2(0.0f, 0.0f);
+    for (int at = threadIdx.x * 4; at < kp; at += 128 * 4) {
+        uint2 part[3];
+        split_four(at < k ? *reinterpret_cast<const float4*>(a + (int64_t)row * lda + at) : make_float4(0.f, 0.f, 0.f, 0.f), part,
+                   wild);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) parts[((int64_t)(i * m + row) * kp + at) / 4] = part[i];
+    }
+    const int any = __syncthreads_or(wild.x != 0.0f || wild.y != 0.0f);                 // (NaN)
+    if (threadIdx.x == 0) wild_x[row] = any;
+}
+
+// One CTA: a tile of up to 128 columns of c and `nx` rows, over groups [z * groups_per, ...) of k.  partial == nullptr: all groups,
+// whose sums meet in c; else group g goes to partial[g][m][n].  map_x: the parts of x.
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x, const float* a, int64_t lda,
+                   const float* __restrict__ w, int64_t ldw, float* c, int64_t ldc, float* partial, int groups_per, int m, int n,
+                   int k, int nx) {
+    extern __shared__ uint8_t raw_shared[];
+    const uint32_t base = (smem_address(raw_shared) + 1023u) & ~1023u;
+    uint8_t* aligned = raw_shared + (base - smem_address(raw_shared));
+    const uint32_t bars = base + STAGES * STAGE_BYTES;
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto done_bar = [&](int s) { return bars + 8u * (STAGES + s); };
+    uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(aligned + STAGES * STAGE_BYTES + BARRIERS * 8);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    volatile uint8_t* wild_rows = reinterpret_cast<volatile uint8_t*>(tmem_base_slot + 4);      // [128] of w, [128] of x
+    int* status = &tvb_gemm_f32_tc_status_word;
+
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int col0 = blockIdx.x * BW, row0 = blockIdx.y * nx;
+    const int k_from = blockIdx.z * groups_per * GROUP, k_to = min(k, k_from + groups_per * GROUP);
+    const int blocks = (k_to - k_from + BK - 1) / BK;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), WORK_WARPS + 1); mbar_init(done_bar(s), 1); }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        prefetch_tensormap(&map_x);
+    }
+    if (threadIdx.x < BW) wild_rows[threadIdx.x] = 0;
+    if (warp == 0) tmem_alloc(smem_address(tmem_base_slot), TMEM_COLS);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_base_slot;
+    // waits of a whole warp: one lane waits with the limit and tells the others
+    auto warp_wait = [&](uint32_t bar, uint32_t parity, int code) {
+        int ready = lane == 0 ? (int)mbar_wait(bar, parity, abort_flag, status, code) : 1;
+        ready = __shfl_sync(0xffffffffu, ready, 0);
+        if (ready)
+            for (int tries = 0; tries < 1024 && !mbar_try(bar, parity); ++tries) {}
+        __syncwarp();
+        return ready != 0;
+    };
+
+    if (warp < WORK_WARPS) {
+        // ---- Operands: 4 k of every 32nd row of w a thread, the next block's values in flight while this one's are split.
+        // Sums: the 32 lanes of tensor memory that the warp's number modulo 4 names, SUM_COLS of the rows of x.
+        // Block b is split while the products of b - 1 run, then the sums of b - 1 are added up.  When those are done, the
+        // stage that b + 1 goes to is free, and a warp that hands b + 1 over has read the accumulator it goes to.
+        const int chunk = threadIdx.x & 15, r0 = threadIdx.x >> 4;
+        const float* w_from = w + (int64_t)(col0 + r0) * ldw + k_from + chunk * 4;
+        const uint32_t w_at = base + (uint32_t)(r0 * 128 + (((chunk >> 1) ^ (r0 & 7)) << 4) + (chunk & 1) * 8);   // (32 rows: the same)
+        float4 held[PASSES];
+        float2 wild = make_float2(0.0f, 0.0f);
+        auto load = [&](int pass, int block) {
+            const bool in = col0 + r0 + pass * ROWS_A_PASS < n && k_from + block * BK + chunk * 4 < k_to;
+            held[pass] = in ? *reinterpret_cast<const float4*>(w_from + (int64_t)(pass * ROWS_A_PASS) * ldw + block * BK)
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        const int quarter = warp & 3, first = (warp >> 2) * SUM_COLS;
+        const int col = col0 + quarter * 32 + lane;
+        const int rows = min(min(nx - first, SUM_COLS), m - row0 - first); // of this warp's sums; none where negative
+        float sum[SUM_COLS];
+#pragma unroll
+        for (int j = 0; j < SUM_COLS; ++j) sum[j] = 0.0f;
+#pragma unroll
+        for (int pass = 0; pass < PASSES; ++pass) load(pass, 0);
+        for (int b = 0; b <= blocks; ++b) {
+            if (b < blocks) {
+#pragma unroll
+                for (int pass = 0; pass < PASSES; ++pass) {
+                    uint2 part[3];
+                    split_four(held[pass], part, wild);
+                    if (b + 1 < blocks) load(pass, b + 1);
+                    const uint32_t at = w_at + (uint32_t)((b & 1) * STAGE_BYTES + pass * ROWS_A_PASS * 128);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};\n" ::"r"(at + (uint32_t)(i * PART_BYTES)), "r"(part[i].x),
+                                     "r"(part[i].y) : "memory");
+                }
+                fence_async_shared();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full_bar(b & 1));
+            }
+            if (b == 0) continue;
+            const int before = b - 1, acc = before & 1;
+            if (!warp_wait(done_bar(acc), (before >> 1) & 1u, GAVE_UP_DONE)) break;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int at = 0; at < SUM_COLS; at += 8) {
+                if (at >= rows) break;
+                uint32_t v[8];
+                tmem_load_8(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * MAX_X + first + at), v);
+                tmem_load_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) sum[at + j] = __fadd_rn(sum[at + j], __uint_as_float(v[j]));
+            }
+            tc_fence_before_sync();
+            if (b % GROUP_BLOCKS != 0 && b != blocks) continue;
+            const int g = before / GROUP_BLOCKS;
+            const int64_t ld = partial ? n : ldc;
+            float* to = (partial ? partial + (int64_t)(blockIdx.z * groups_per + g) * m * n : c) + (int64_t)(row0 + first) * ld + col;
+            if (col < n) {
+#pragma unroll
+                for (int j = 0; j < SUM_COLS; ++j) {
+                    if (j < rows) *to = !partial && g > 0 ? __fadd_rn(*to, sum[j]) : sum[j];        // (this thread's own sum so far)
+                    to += ld;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < SUM_COLS; ++j) sum[j] = 0.0f;
+        }
+        if (wild.x != 0.0f || wild.y != 0.0f)                              // (NaN: of one of the thread's rows)
+#pragma unroll
+            for (int pass = 0; pass < PASSES; ++pass) wild_rows[r0 + pass * ROWS_A_PASS] = 1;
+    } else {
+        // ---- copies of x, a block ahead, and products: of a block the smallest first
+        const uint32_t idesc = instruction_descriptor_bf16(BW, nx, false);
+        auto copy = [&](int b) {
+            if (elect_lane()) {
+                const uint32_t at = base + (b & 1) * STAGE_BYTES + 3 * PART_BYTES;
+                mbar_arrive_expect(full_bar(b & 1), 3u * (uint32_t)nx * BK * 2);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) tma_load_3d(at + i * PART_BYTES, &map_x, k_from + b * BK, row0, i, full_bar(b & 1));
+            }
+            __syncwarp();
+        };
+        pdl_wait();
+        copy(0);
+        if (blocks > 1) copy(1);
+        for (int b = 0; b < blocks; ++b) {
+            if (!warp_wait(full_bar(b & 1), (b >> 1) & 1u, GAVE_UP_FULL)) break;
+            tc_fence_after_sync();
+            if (elect_lane()) {
+                const uint32_t w_at = base + (b & 1) * STAGE_BYTES, x_at = w_at + 3 * PART_BYTES;
+                const uint32_t d_tmem = tmem_base + (uint32_t)((b & 1) * MAX_X);
+                constexpr int W_PART[6] = {2, 0, 1, 1, 0, 0}, X_PART[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+                for (int p = 0; p < 6; ++p) {
+                    const uint64_t w_desc = tile_descriptor(w_at + W_PART[p] * PART_BYTES);
+                    const uint64_t x_desc = tile_descriptor(x_at + X_PART[p] * PART_BYTES);
+#pragma unroll
+                    for (int kk = 0; kk < BK / UMMA_K; ++kk) tc_mma(d_tmem, w_desc + 2u * kk, x_desc + 2u * kk, idesc, (p | kk) != 0);
+                }
+                tc_commit(done_bar(b & 1));
+            }
+            __syncwarp();
+            if (b > 0 && b + 1 < blocks) {
+                if (!warp_wait(done_bar((b - 1) & 1), ((b - 1) >> 1) & 1u, GAVE_UP_FREE)) break;
+                copy(b + 1);
+            }
+        }
+    }
+
+    tc_fence_before_sync();
+    __syncthreads();
+    const bool gave_up = *abort_flag != 0;
+    if (gave_up) {
+        // copies or products may still be in flight from and to this CTA's memory: give them time
+        const long long started = clock64();
+        while (clock64() - started < 400000) __nanosleep(1000);
+    }
+    pdl_wait();
+    if (threadIdx.x >= BW && threadIdx.x < 2 * BW) {
+        const int row = threadIdx.x - BW;
+        wild_rows[threadIdx.x] = row < nx && row0 + row < m && *reinterpret_cast<const volatile int*>(wild_x + row0 + row) != 0;
+    }
+    const int wild = threadIdx.x < 2 * BW && wild_rows[threadIdx.x] != 0;
+    if (__syncthreads_or(wild) && !gave_up) {
+        // of the rows of w that a thread has marked, those that hold such a value
+        for (int r = warp; r < BW; r += THREADS / 32) {
+            if (!wild_rows[r]) continue;
+            bool found = false;
+            for (int at = k_from + lane; at < k_to && col0 + r < n; at += 32)
+                found |= ((__float_as_uint(w[(int64_t)(col0 + r) * ldw + at]) + 0x8000u) & 0x7fffffffu) >= 0x7f800000u;
+            found = __any_sync(0xffffffffu, found);
+            if (lane == 0) wild_rows[r] = found;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < BW * nx; i += THREADS) {
+            const int local_col = i % BW, local_row = i / BW, col = col0 + local_col, row = row0 + local_row;
+            if (col >= n || row >= m || !(wild_rows[local_col] | wild_rows[BW + local_row])) continue;
+            float total = 0.0f;
+            for (int g = 0; k_from + g * GROUP < k_to; ++g) {
+                const float sum = plain_sum(a + (int64_t)row * lda, w + (int64_t)col * ldw, k_from + g * GROUP,
+                                            min(k_to, k_from + (g + 1) * GROUP));
+                if (partial) partial[((int64_t)(blockIdx.z * groups_per + g) * m + row) * n + col] = sum;
+                total = g == 0 ? sum : __fadd_rn(total, sum);
+            }
+            if (!partial) c[(int64_t)row * ldc + col] = total;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after_sync();
+        tmem_free(tmem_base, TMEM_COLS);
+    }
+}
+
+// c = the sum of the groups' partial products, in ascending order
+__global__ void __launch_bounds__(256)
+fold_groups_kernel(const float* __restrict__ partial, int groups, float* __restrict__ c, int64_t ldc, int m, int n) {
+    const int64_t size = (int64_t)m * n;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += (int64_t)gridDim.x * blockDim.x) {
+        float total = partial[i];
+        for (int g = 1; g < groups; ++g) total = __fadd_rn(total, partial[g * size + i]);
+        c[(i / n) * ldc + i % n] = total;
+    }
+}
+
+struct Plan { int nx, tiles_x, groups, groups_per, splits; };
+
+constexpr long long SCRATCH_FLOATS = 16LL << 20;      // the most that partial sums take
+
+Plan plan_of(int m, int n, int k, int sms) {
+    Plan best{};
+    best.groups = (k + GROUP - 1) / GROUP;
+    const long long tiles_w = (n + BW - 1) / BW;
+    const int fewest = (m + MAX_X - 1) / MAX_X;
+    double least = 0.0;
+    for (int tiles = fewest; tiles <= fewest + 4 && tiles <= (m + 15) / 16; ++tiles) {
+        const int nx = ((m + tiles - 1) / tiles + 15) / 16 * 16, tiles_x = (m + nx - 1) / nx;
+        const double block_us = 1.42 + 0.0035 * nx;
+        for (int per = best.groups; per >= 1; --per) {
+            const int splits = (best.groups + per - 1) / per;
+            if (splits > 1 && ((long long)best.groups * m * n > SCRATCH_FLOATS || splits > 65535)) break;
+            const long long waves = (tiles_w * tiles_x * splits + sms - 1) / sms;
+            const double us = waves * (std::min(per * GROUP, k) / BK * block_us + 4.0) +
+                              (splits > 1 ? 3.0 + 8.0 * best.groups * m * n / 6e6 : 0.0);
+            if (best.nx == 0 || us < least) {
+                least = us;
+                best.nx = nx; best.tiles_x = tiles_x; best.groups_per = per; best.splits = splits;
+            }
+        }
+    }
+    return best;
+}
+
+// Scratch of a product: partial sums, the parts of x, and a word a row of x.
+long long padded_k(int k) { return (k + BK - 1) / BK * BK; }
+long long sum_bytes(const Plan& plan, int m, int n) {
+    return plan.splits > 1 ? ((long long)plan.groups * m * n * 4 + 127) / 128 * 128 : 0;
+}
+
+}  // namespace
+
+// 0, or which wait gave up in some launch since the last call (1 operands, 2 and 3 products); reading clears it.
+// Synchronises the device.
+extern "C" int tvb_gemm_f32_tc_status() {
+    int value = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&value, tvb_gemm_f32_tc_status_word, sizeof(int)) != cudaSuccess) return -1;
+    if (value != 0) cudaMemcpyToSymbol(tvb_gemm_f32_tc_status_word, &zero, sizeof(int));
+    return value;
+}
+
+extern "C" long long tvb_gemm_f32_tc_scratch_bytes(int m, int n, int k) {
+    const int sms = tvb_sm_count();
+    if (m <= 0 || n <= 0 || k <= 0 || sms <= 0) return 0;
+    return sum_bytes(plan_of(m, n, k, sms), m, n) + 3 * m * padded_k(k) * 2 + 4ll * m;
+}
+
+// kernels that a product launches
+extern "C" int tvb_gemm_f32_tc_launches(int m, int n, int k) {
+    const int sms = tvb_sm_count();
+    if (m <= 0 || n <= 0 || k <= 0 || sms <= 0) return 0;
+    return plan_of(m, n, k, sms).splits > 1 ? 3 : 2;
+}
+
+// c[m, n] = a . w^T; rows of a and w on 16-byte boundaries.  scratch: tvb_gemm_f32_tc_scratch_bytes, on a 128-byte
+// boundary.  nx, splits: 0, or force the rows of a tile and the pieces of k.
+extern "C" int tvb_gemm_f32_tc(const float* a, long long lda, const float* w, long long ldw, float* c, long long ldc, int m,
+                               int n, int k, uint8_t* scratch, int nx, int splits, int pdl, void* stream) {
+    if (m <= 0 || n <= 0) return 0;
+    if (k <= 0 || k % 4 || lda % 4 || ldw % 4 || !scratch ||
+        ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) || (reinterpret_cast<uintptr_t>(scratch) & 127))
+        return TVB_BAD_ARGUMENT;
+    const int sms = tvb_sm_count();
+    if (sms <= 0) return (int)cudaErrorInvalidDevice;
+    Plan plan = plan_of(m, n, k, sms);
+    if (nx > 0) {
+        plan.nx = nx; plan.tiles_x = (m + nx - 1) / nx;
+        plan.groups_per = (plan.groups + splits - 1) / splits; plan.splits = (plan.groups + plan.groups_per - 1) / plan.groups_per;
+    }
+    if (plan.tiles_x > 65535) return TVB_BAD_ARGUMENT;
+    float* partial = plan.splits > 1 ? reinterpret_cast<float*>(scratch) : nullptr;
+    uint8_t* parts = scratch + sum_bytes(plan, m, n);
+    const long long kp = padded_k(k);
+    int* wild_x = reinterpret_cast<int*>(parts + 3 * m * kp * 2);
+    CUtensorMap map_x;
+    {
+        const cuuint64_t dims[3] = {(cuuint64_t)kp, (cuuint64_t)m, 3};
+        const cuuint64_t strides[2] = {(cuuint64_t)kp * 2, (cuuint64_t)(m * kp * 2)};
+        const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)plan.nx, 1};
+        if (!tvb_make_map(&map_x, parts, 3, dims, strides, box)) return (int)cudaErrorNotSupported;
+    }
+    cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    cudaStream_t s = (cudaStream_t)stream;
+    split_rows_kernel<<<m, 128, 0, s>>>(a, lda, reinterpret_cast<uint2*>(parts), wild_x, m, k, (int)kp);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+    TvbLaunch launch(dim3((n + BW - 1) / BW, plan.tiles_x, plan.splits), dim3(THREADS), SHARED_BYTES, s, pdl);
+    e = cudaLaunchKernelEx(&launch.config, gemm_f32_tc_kernel, map_x, (const int*)wild_x, a, (int64_t)lda, w, (int64_t)ldw, c,
+                           (int64_t)ldc, partial, plan.groups_per, m, n, k, plan.nx);
+    if (e != cudaSuccess) return (int)e;
+    if (plan.splits > 1) {
+        const int blocks = (int)std::min<long long>(((long long)m * n + 255) / 256, 8LL * sms);
+        fold_groups_kernel<<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n);
+    }
+    return tvb_last_error();
+}

@@ -1884,6 +1884,54 @@ def gemm_f32_scratch_floats(m: int, n: int, k: int) -> int:
     return _fn("gemm_simt", "tvb_gemm_f32_scratch_floats", [c_int, c_int, c_int], c_longlong)(m, n, k)
 
 
+def gemm_f32_tc_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether :func:`gemm_f32_tc` takes this product: float32, rows contiguous and on 16-byte boundaries, k a
+    multiple of 4."""
+    return (a.dtype == torch.float32 and w.dtype == torch.float32 and a.dim() == 2 and w.dim() == 2
+            and a.shape[1] == w.shape[1] and a.shape[1] > 0 and a.shape[1] % 4 == 0 and a.stride(1) == 1 and w.stride(1) == 1
+            and a.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """a [m, k] . w [n, k]^T of float32 operands on the tensor cores, each operand as three bfloat16 whose products are
+    added up to float32 sums; the order of a sum over k depends on k alone."""
+    _need_cuda(a, w)
+    if not gemm_f32_tc_takes(a, w):
+        raise KernelError("gemm_f32_tc wants float32 a [m, k] and w [n, k] with contiguous, 16-byte aligned rows, "
+                          "k a multiple of 4")
+    m, k = a.shape
+    n = w.shape[0]
+    if out is None:
+        out = torch.empty((m, n), dtype=torch.float32, device=a.device)
+    elif out.dtype != torch.float32 or out.shape != (m, n) or (out.stride(1) != 1 and n > 1):
+        raise KernelError("gemm_f32_tc: out must be float32 [m, n] with contiguous rows")
+    if m == 0 or n == 0:
+        return out
+    sizes = [c_int, c_int, c_int]
+    # the parts of a, and partial sums where k is cut
+    scratch = torch.empty(_fn("gemm_f32_tc", "tvb_gemm_f32_tc_scratch_bytes", sizes, c_longlong)(m, n, k), dtype=torch.uint8,
+                          device=a.device)
+    fn = _fn("gemm_f32_tc", "tvb_gemm_f32_tc",
+             [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_int,
+              c_int, c_int, c_void_p])
+    global _gemm_tc_unchecked, _gemm_f32_tc_used
+    _check(fn(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), m, n, k,
+              scratch.data_ptr(), 0, 0, _pdl("gemm"), _stream()), "gemm_f32_tc",
+           _fn("gemm_f32_tc", "tvb_gemm_f32_tc_launches", sizes)(m, n, k))
+    _gemm_tc_unchecked = _gemm_f32_tc_used = True
+    _guarded_counts[0] += 1
+    return out
+
+
+_gemm_f32_tc_used = False
+
+
+def gemm_f32_tc_status() -> int:
+    """0, or which bounded wait of a gemm_f32_tc launch gave up since the last call.  Synchronises the device; reading
+    clears the record."""
+    return _fn("gemm_f32_tc", "tvb_gemm_f32_tc_status", [])()
+
+
 # ------------------------------------------------------------------- sampling
 def sample_rows(logits: torch.Tensor, packed: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """One token per row of logits [rows, vocab].  ``packed`` is int32 [7, capacity >= rows],
@@ -2462,7 +2510,7 @@ _guarded_counts = [0, 0]
 
 
 def guarded_launch_counts() -> tuple[int, int]:
-    """How often (gemm_tc or gemm_stream, attention_prefill_tc), the kernels with bounded waits, were launched
+    """How often (gemm_tc, gemm_stream or gemm_f32_tc, attention_prefill_tc), the kernels with bounded waits, were launched
     through this module so far.  A caller that records a step into a CUDA graph compares the
     counts around one pass of the step and hands what it finds to :func:`note_guarded_launches`
     at every replay: a replay launches the kernels without passing through this module."""
@@ -2489,6 +2537,11 @@ def check_finished_launches() -> None:
             status = gemm_stream_status()
             if status:
                 raise KernelError(f"gemm_stream: a wait inside the kernel ran out (code {status}); "
+                                  "the results of this step are not valid")
+        if _gemm_f32_tc_used:
+            status = gemm_f32_tc_status()
+            if status:
+                raise KernelError(f"gemm_f32_tc: a wait inside the kernel ran out (code {status}); "
                                   "the results of this step are not valid")
     if _attention_tc_unchecked:
         status = attention_prefill_tc_status()

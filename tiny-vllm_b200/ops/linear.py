@@ -1,6 +1,7 @@
 """x . W^T for the parts, by storage dtype.
 
-float32: the package's own float32-core kernels (true 32-bit; the order of a sum depends on k alone).
+float32: the package's own kernels, true 32-bit: up to F32_CORE_ROWS rows on the float32 cores, more on the tensor
+cores with every operand as three bfloat16 (each of the two gives a row the same bits whatever else is in the batch).
 bfloat16: the tensor-core kernels of this package where they take the shape,
 else cuBLAS through ``torch.nn.functional.linear``, which is what the
 reference's engine calls for every projection (tinyvllm/layers.py:84-85).
@@ -25,10 +26,22 @@ def linear(x: torch.Tensor, weight: torch.Tensor, *, out_dtype: torch.dtype | No
     if x.dtype == torch.float32:
         if out_dtype != torch.float32:
             raise kernels.KernelError("a float32 product has a float32 result")
-        return kernels.gemm_nt_simt(x, weight, out=out)
+        return _linear_f32(x, weight, out)
     from . import gemm
 
     return gemm.linear_bf16(x, weight, out_dtype=out_dtype, out=out)
+
+
+# Rows up to which a float32 product stays on the float32 cores: the tensor-core kernel takes 28 to 31 us for a layer's
+# products at any number of rows up to 128 (a CTA walks 1,024 k in 16 steps of 1.4 us), the float32 cores 16 to 24 us
+# for 32 rows, 29 to 42 us for 48.
+F32_CORE_ROWS = 32
+
+
+def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None) -> torch.Tensor:
+    if x.shape[0] > F32_CORE_ROWS and kernels.gemm_f32_tc_takes(x, weight):
+        return kernels.gemm_f32_tc(x, weight, out=out)
+    return kernels.gemm_nt_simt(x, weight, out=out)
 
 
 def linear_silu(x: torch.Tensor, gate_up_weight: torch.Tensor) -> torch.Tensor:
@@ -36,7 +49,7 @@ def linear_silu(x: torch.Tensor, gate_up_weight: torch.Tensor) -> torch.Tensor:
     if not x.is_cuda:
         raise kernels.KernelError("linear_silu runs on CUDA tensors only; there is no CPU path")
     if x.dtype == torch.float32:
-        return kernels.silu_mul(kernels.gemm_nt_simt(x, gate_up_weight))
+        return kernels.silu_mul(_linear_f32(x, gate_up_weight, None))
     from . import gemm
 
     return gemm.linear_silu_bf16(x, gate_up_weight)
