@@ -1,0 +1,45 @@
+"""The RMS norm of float32 rows: the register form at the edges of its widths, the general one beside it, and weights that
+the launch before writes (of the norm and of products of a few rows)."""
+
+import pytest
+import torch
+
+from tinyvllm_b200.ops import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("width", [4, 31, 36, 1020, 1024, 1028, 4096, 4100, 8192, 8196])
+@pytest.mark.parametrize("constant", [False, True])
+def test_against_64_bits(width, constant):
+    generator = torch.Generator(device="cuda").manual_seed(width)
+    x, r = (torch.randn(37, width, generator=generator, device="cuda") for _ in range(2))
+    weight = torch.randn(width, generator=generator, device="cuda")
+    got, stream = kernels.rms_norm(x, weight, 1e-6, residual=r, weight_constant=constant)
+    assert torch.equal(stream, x + r)
+    wide = (x + r).double()
+    want = wide / (wide.square().mean(1, keepdim=True) + 1e-6).sqrt() * weight.double()
+    # the sum of squares over chains of at most 16 and 9 halvings, its root, the quotient and two products
+    assert ((got.double() - want).abs() <= 32 * 2.0 ** -24 * want.abs()).all()
+    rows = torch.tensor([36, 0, 5], dtype=torch.int32, device="cuda")
+    assert torch.equal(kernels.rms_norm(x + r, weight, 1e-6, rows=rows), got[rows.long()])
+    shifted = torch.empty(37 * width + 1, device="cuda")[1:].view(37, width).copy_(x + r)          # off the 16-byte boundary
+    assert ((kernels.rms_norm(shifted, weight, 1e-6).double() - want).abs() <= 32 * 2.0 ** -24 * want.abs()).all()
+
+
+@pytest.mark.parametrize("width", [64, 1024, 4096])
+def test_weights_and_products_of_the_launch_before_are_awaited(width):
+    generator = torch.Generator(device="cuda").manual_seed(width)
+    x = torch.randn(3000, width, generator=generator, device="cuda")
+    rows = torch.randn(5, width, generator=generator, device="cuda")
+    made = torch.empty_like(x)
+    for turn in range(40):
+        made.fill_(50.0)                            # what a reader ahead of the store would see
+        weight = torch.randn(width, generator=generator, device="cuda")
+        kernels.rms_norm(x, weight, 1e-6, out=made)
+        got = kernels.rms_norm(rows, made[2999 - turn], 1e-6)
+        assert torch.equal(got, kernels.rms_norm(rows, made[2999 - turn].clone(), 1e-6)), turn
+        made.fill_(50.0)
+        kernels.rms_norm(x, weight, 1e-6, out=made)
+        got = kernels.gemm_nt_simt(rows, made[2900:])                # a weight that the launch before writes
+        assert torch.equal(got, kernels.gemm_nt_simt(rows, made[2900:].clone())), turn

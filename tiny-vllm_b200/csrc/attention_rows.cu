@@ -305,12 +305,13 @@ __global__ void paged_attention_rows_kernel(
 }
 
 template <typename T, int DIMS>
-__global__ void merge_attention_rows_kernel(const float* __restrict__ scratch, int max_chunks,
-                                            const int* __restrict__ token_row,
-                                            const int* __restrict__ positions, T* __restrict__ out,
+__global__ void merge_attention_rows_kernel(const float* scratch, int max_chunks,      // (plain: read behind the wait)
+                                            const int* token_row, const int* positions, T* out,
                                             int64_t out_token_stride, const T* gate, int64_t gate_token_stride,
                                             int tokens, int num_q, int head_dim, int window, int keep_first,
                                             RowExtras extras) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * ATTN_WARPS + warp;
     if (row >= (int64_t)tokens * num_q) return;
@@ -396,7 +397,7 @@ static void launch_rows(const void* q, long long q_token_stride, const void* key
 // lets them be a part of the key rows.
 // `bias_table` (float32 [bias_rows, num_q], or null): table[min(p - j, bias_rows - 1), h] is added to the
 // score of key j; `segment` > 0: the query at p sees only keys from p - p % segment on; `softcap` > 0: a scaled
-// score s becomes softcap * tanh(s / softcap).
+// score s becomes softcap * tanh(s / softcap).  `pdl`: plain float32 heads cut into chunks are launched programmatically.
 extern "C" int tvb_attention_rows_masked(const void* q, long long q_token_stride, const void* key_cache,
                                          const void* value_cache, long long value_stride, const int* block_tables,
                                          int table_stride, const int* token_row, const int* positions, void* out,
@@ -405,7 +406,7 @@ extern "C" int tvb_attention_rows_masked(const void* q, long long q_token_stride
                                          const float* bias_table, int bias_rows, int segment,
                                          float* scratch, int max_chunks, int tokens, int num_q, int num_kv,
                                          int head_dim, int value_dim, int page_size, int window, int keep_first,
-                                         float scale, float softcap, int dtype, void* stream) {
+                                         float scale, float softcap, int dtype, int pdl, void* stream) {
     if (tokens <= 0) return 0;
     if (segment < 0 || (bias_table && bias_rows <= 0)) return TVB_BAD_ARGUMENT;
     if (head_dim <= 0 || head_dim > 32 * ATTN_WIDE_DIMS || value_dim <= 0 || value_dim > 32 * ATTN_WIDE_DIMS ||
@@ -428,13 +429,15 @@ extern "C" int tvb_attention_rows_masked(const void* q, long long q_token_stride
         ((reinterpret_cast<uintptr_t>(key_cache) | reinterpret_cast<uintptr_t>(value_cache)) & 15) == 0) {
         const F32Args args{(const float*)q, q_token_stride, (const float*)key_cache, (const float*)value_cache, block_tables,
                            table_stride, token_row, positions, (float*)out, out_token_stride, scratch, max_chunks, tokens,
-                           num_q, num_kv, page_size, window, scale};
+                           num_q, num_kv, page_size, window, scale, pdl};
         const int status = launch_f32_of(head_dim, group, args, s);
         if (status != 0 || max_chunks == 0) return status;
-        merge_attention_rows_kernel<float, ATTN_MAX_DIMS><<<(unsigned)blocks, ATTN_WARPS * 32, 0, s>>>(
-            scratch, max_chunks, token_row, positions, (float*)out, out_token_stride, nullptr, 0, tokens, num_q, value_dim,
-            window, 0, extras);
-        return tvb_last_error();
+        TvbLaunch launch(dim3((unsigned)blocks), dim3(ATTN_WARPS * 32), 0, s, pdl);
+        const cudaError_t e = cudaLaunchKernelEx(
+            &launch.config, merge_attention_rows_kernel<float, ATTN_MAX_DIMS>, (const float*)scratch, max_chunks, token_row,
+            positions, (float*)out, (int64_t)out_token_stride, (const float*)nullptr, (int64_t)0, tokens, num_q, value_dim, window,
+            0, extras);
+        return e == cudaSuccess ? tvb_last_error() : (int)e;
     }
 #define LAUNCH_ROWS(T, DIMS)                                                                             \
     launch_rows<T, DIMS>(q, q_token_stride, key_cache, value_cache, block_tables, table_stride, token_row, \
@@ -460,7 +463,7 @@ extern "C" int tvb_attention_rows_biased(const void* q, long long q_token_stride
                                      table_stride, token_row, positions, out, out_token_stride, gate,
                                      gate_token_stride, gate_per_head, slopes, sinks, nullptr, 0, 0, scratch,
                                      max_chunks, tokens, num_q, num_kv, head_dim, value_dim, page_size, window,
-                                     keep_first, scale, 0.0f, dtype, stream);
+                                     keep_first, scale, 0.0f, dtype, 0, stream);
 }
 
 extern "C" int tvb_attention_rows_general(const void* q, long long q_token_stride, const void* key_cache,

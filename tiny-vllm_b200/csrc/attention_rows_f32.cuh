@@ -47,6 +47,7 @@ struct F32Args {
     float* scratch;                        // mode split: the partials
     int max_chunks, tokens, num_q, num_kv, page_size, window;
     float scale;
+    int pdl;                               // the launch for single tokens in mode split
 };
 
 // Whether `token` is attended in a tile: its run of tokens of one request, within the tile of `tile_tokens` it
@@ -208,6 +209,8 @@ __global__ void __launch_bounds__(F32_THREADS) attention_f32_token_kernel(F32Arg
     extern __shared__ __align__(16) float f32_shared[];
     __shared__ F32Shared sh;
     const int tid = threadIdx.x, token = blockIdx.x / a.num_kv, kv_head = blockIdx.x % a.num_kv, chunk = blockIdx.y;
+    pdl_launch_dependents();
+    pdl_wait();
     const int position = a.positions[token], request = a.token_row[token];
     if (request < 0 || position < 0) {                             // padding row of a captured batch
         if (chunk == 0) f32_zero_token<D, GROUP>(a, token, kv_head);
@@ -550,7 +553,9 @@ static int launch_f32(const F32Args& a, cudaStream_t s) {
     auto kernel = attention_f32_token_kernel<D, GROUP>;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, token_shared);
     if (e != cudaSuccess) return (int)e;
-    kernel<<<dim3((unsigned)(a.tokens * a.num_kv), a.max_chunks), F32_THREADS, token_shared, s>>>(a, tiled ? TOKENS : 0);
+    TvbLaunch launch(dim3((unsigned)(a.tokens * a.num_kv), a.max_chunks), dim3(F32_THREADS), token_shared, s, a.pdl);
+    e = cudaLaunchKernelEx(&launch.config, kernel, a, tiled ? TOKENS : 0);
+    if (e != cudaSuccess) return (int)e;
     if (tiled) {
         auto tile_kernel = attention_f32_tile_kernel<D, GROUP>;
         e = cudaFuncSetAttribute(tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_shared);

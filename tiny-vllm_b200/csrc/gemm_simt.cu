@@ -19,6 +19,9 @@
 // 1,024 x 3,072 229 / 9.5, 151,936 x 1,024 709 / 150 (one row: 703 / 118, 5.3 TB/s); 64 rows 6,144 x 1,024 80 / 58;
 // 677 rows 4,096 x 1,024 251 / 176, 1,024 x 2,048 215 / 93, 6,144 x 1,024 390 / 260 (33 TFLOP/s; 2,048 rows 37.5: three
 // 64-bit operands keep the packed instruction at about 44 on this part, scalar ones on the same layout were slower).
+// In a decode step of 4 rows (28 layers of the 0.6B sizes) the products of up to 8 rows are launched programmatically and ask
+// for their first stages (64 KB a CTA of 16 columns) while the kernel before runs: with the small kernels between them
+// launched the same way, and the norm below, 1,780 to 1,500 us a step.
 // Error against 64-bit sums (2-norm): 5.7e-7 at k = 1,024 and 9.9e-7 at k = 3,072 before, 1.6e-7 at both.
 //
 // bfloat16 operands (sizes the tensor-core products do not take): one plain tile kernel, one ascending chain.
@@ -123,8 +126,8 @@ __device__ __forceinline__ void copy_four(float* dst, const float* row, int k0, 
 
 template <int ROWS, int COLS, int STAGES, bool ALIGNED>
 __global__ void __launch_bounds__(COLS * FEW_SEGMENTS)
-gemm_f32_few_kernel(const float* __restrict__ a, int64_t lda, const float* __restrict__ w, int64_t ldw,
-                    float* __restrict__ c, int64_t ldc, int m, int n, int k) {
+gemm_f32_few_kernel(const float* a, int64_t lda, const float* w, int64_t ldw, float* c, int64_t ldc, int m, int n, int k,
+                    int w_constant) {
     constexpr int THREADS = COLS * FEW_SEGMENTS;
     static_assert(ROWS * COLS <= THREADS, "one thread folds one output");
     extern __shared__ __align__(16) float few_shared[];
@@ -158,17 +161,23 @@ gemm_f32_few_kernel(const float* __restrict__ a, int64_t lda, const float* __res
         load_stage = load_stage + 1 == STAGES ? 0 : load_stage + 1;
         if (++load_chunk == chunks) { load_chunk = 0; load_tile += gridDim.x; }
     };
+    // Under programmatic dependent launch this kernel may run beside the one before it, and lets the next one do the same.
+    // A weight that no kernel in flight writes is asked for at once, before the wait for the rows of x.
+    pdl_launch_dependents();
+    if (!w_constant) pdl_wait();
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s)
+        if (s < items) load();
+    if (w_constant) pdl_wait();
 #pragma unroll
     for (int row = 0; row < ROWS; ++row) {
         const float* from = a + (int64_t)min(row, m - 1) * lda;
         for (int q = tid; q < segments * (SEGMENT / 4); q += THREADS)
             copy_four<ALIGNED>(x + row * x_row + (q / (SEGMENT / 4)) * X_SEGMENT + (q % (SEGMENT / 4)) * 4, from, q * 4, k, row < m);
     }
+    // x and the first stages are one group, the oldest; the others of the ring's start are empty
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < items) load();
-        cp_async_commit();
-    }
+    for (int s = 0; s < STAGES - 1; ++s) cp_async_commit();
     float total = 0.0f;
     int tile = blockIdx.x, chunk = 0, at_stage = 0;
     for (int item = 0; item < items; ++item) {
@@ -402,7 +411,7 @@ static TilePlan tile_plan(int m, int n, int k) {
 
 template <int ROWS, int COLS, int STAGES, bool ALIGNED>
 static int launch_few(const float* a, long long lda, const float* w, long long ldw, float* c, long long ldc, int m, int n,
-                      int k, cudaStream_t s) {
+                      int k, int pdl, int w_constant, cudaStream_t s) {
     auto kernel = gemm_f32_few_kernel<ROWS, COLS, STAGES, ALIGNED>;
     const int shared = (int)few_shared_bytes(ROWS, COLS, STAGES, k);
     // (one limit for all k: a smaller one could come between another thread's limit and its launch)
@@ -412,16 +421,17 @@ static int launch_few(const float* a, long long lda, const float* w, long long l
     const int tiles = (n + COLS - 1) / COLS;
     // as many CTAs as run at once, each with the same number of tiles but for one
     const int turns = (tiles + SMS * resident - 1) / (SMS * resident);
-    kernel<<<(tiles + turns - 1) / turns, COLS * FEW_SEGMENTS, shared, s>>>(a, lda, w, ldw, c, ldc, m, n, k);
-    return tvb_last_error();
+    TvbLaunch launch(dim3((tiles + turns - 1) / turns), dim3(COLS * FEW_SEGMENTS), shared, s, pdl);
+    e = cudaLaunchKernelEx(&launch.config, kernel, a, (int64_t)lda, w, (int64_t)ldw, c, (int64_t)ldc, m, n, k, w_constant);
+    return e == cudaSuccess ? tvb_last_error() : (int)e;
 }
 
 template <int ROWS, bool ALIGNED>
 static int few_of(const float* a, long long lda, const float* w, long long ldw, float* c, long long ldc, int m, int n, int k,
-                  cudaStream_t s) {
-    if (few_columns(n) == 16) return launch_few<ROWS, 16, 2, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, s);
-    if (few_shared_bytes(ROWS, 8, 3, k) <= SHARED_LIMIT) return launch_few<ROWS, 8, 3, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, s);
-    return launch_few<ROWS, 8, 2, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, s);
+                  int pdl, int w_constant, cudaStream_t s) {
+    if (few_columns(n) == 16) return launch_few<ROWS, 16, 2, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, pdl, w_constant, s);
+    if (few_shared_bytes(ROWS, 8, 3, k) <= SHARED_LIMIT) return launch_few<ROWS, 8, 3, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, pdl, w_constant, s);
+    return launch_few<ROWS, 8, 2, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, pdl, w_constant, s);
 }
 
 template <int BM, int TM, bool ALIGNED>
@@ -450,13 +460,13 @@ static int launch_tiles(const float* a, long long lda, const float* w, long long
 
 template <bool ALIGNED>
 static int gemm_f32(const float* a, long long lda, const float* w, long long ldw, float* c, long long ldc, float* partial,
-                    int m, int n, int k, cudaStream_t s) {
+                    int m, int n, int k, int pdl, int w_constant, cudaStream_t s) {
     if (takes_few(m, n, k)) {
         switch (few_template_rows(m)) {
-            case 1: return few_of<1, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, s);
-            case 2: return few_of<2, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, s);
-            case 4: return few_of<4, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, s);
-            default: return few_of<8, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, s);
+            case 1: return few_of<1, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, pdl, w_constant, s);
+            case 2: return few_of<2, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, pdl, w_constant, s);
+            case 4: return few_of<4, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, pdl, w_constant, s);
+            default: return few_of<8, ALIGNED>(a, lda, w, ldw, c, ldc, m, n, k, pdl, w_constant, s);
         }
     }
     const TilePlan plan = tile_plan(m, n, k);
@@ -482,18 +492,19 @@ extern "C" int tvb_gemm_f32_launches(int m, int n, int k) {
 }
 
 // in_dtype: type of A and W; out_dtype: type of C (float32 output from bfloat16
-// inputs serves the logits); scratch: tvb_gemm_f32_scratch_floats floats, for float32 operands.
+// inputs serves the logits); scratch: tvb_gemm_f32_scratch_floats floats, for float32 operands.  pdl, w_constant: up to
+// 8 rows of float32 run beside the end of the kernel before, which does not write w.
 extern "C" int tvb_gemm_nt_simt(const void* a, long long lda, const void* w, long long ldw, void* c,
                                 long long ldc, int m, int n, int k, int in_dtype, int out_dtype, float* scratch,
-                                void* stream) {
+                                int pdl, int w_constant, void* stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return TVB_BAD_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
     if (in_dtype == TVB_F32 && out_dtype == TVB_F32) {
         const bool aligned = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
                              ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
-        return aligned ? gemm_f32<true>((const float*)a, lda, (const float*)w, ldw, (float*)c, ldc, scratch, m, n, k, s)
-                       : gemm_f32<false>((const float*)a, lda, (const float*)w, ldw, (float*)c, ldc, scratch, m, n, k, s);
+        return aligned ? gemm_f32<true>((const float*)a, lda, (const float*)w, ldw, (float*)c, ldc, scratch, m, n, k, pdl, w_constant, s)
+                       : gemm_f32<false>((const float*)a, lda, (const float*)w, ldw, (float*)c, ldc, scratch, m, n, k, pdl, w_constant, s);
     }
     dim3 grid((n + TILE_N - 1) / TILE_N, (m + TILE_M - 1) / TILE_M);
     if (grid.y > 65535) return TVB_BAD_ARGUMENT;

@@ -19,7 +19,7 @@ from . import kernels
 def linear(x: torch.Tensor, weight: torch.Tensor, *, out_dtype: torch.dtype | None = None,
            out: torch.Tensor | None = None) -> torch.Tensor:
     """x [m, k] times weight [n, k] transposed; the result has ``out_dtype``
-    (default: the dtype of x)."""
+    (default: the dtype of x).  ``weight`` is a parameter, which the kernels may read before the one before them ends."""
     if not x.is_cuda:
         raise kernels.KernelError("linear runs on CUDA tensors only; there is no CPU path")
     out_dtype = out_dtype or x.dtype
@@ -41,7 +41,7 @@ F32_CORE_ROWS = 32
 def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None) -> torch.Tensor:
     if x.shape[0] > F32_CORE_ROWS and kernels.gemm_f32_tc_takes(x, weight):
         return kernels.gemm_f32_tc(x, weight, out=out)
-    return kernels.gemm_nt_simt(x, weight, out=out)
+    return kernels.gemm_nt_simt(x, weight, out=out, weight_constant=True)
 
 
 def linear_silu(x: torch.Tensor, gate_up_weight: torch.Tensor) -> torch.Tensor:
