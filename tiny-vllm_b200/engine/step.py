@@ -85,6 +85,7 @@ class StepContext:
                                          # same signature differ in the contents of their tensors only)
     arena: torch.Tensor | None = None    # the int32 tensor all the fields above are views of
     shared: dict = field(default_factory=dict)   # what a layer of this step hands on to later layers
+    side_stream: object = None                   # while the step is recorded: a stream for a branch beside the main one
 
     def writes_cache(self, run: int) -> bool:
         return self.cache_sources[run] is None
@@ -150,6 +151,7 @@ class StepRunner:
         self._step_seen: dict[tuple, int] = {}
         self._step_graph_pool = None
         self._step_graph_stream = None
+        self._step_graph_side = None
         self._step_count = 0
         self._last_capture_at = -(1 << 30)
         self.decode_splits = attention_ops.decode_splits(self.max_model_len)
@@ -415,6 +417,7 @@ class StepRunner:
         runner stays eager from then on and the step's eager logits stand."""
         if self._step_graph_stream is None:
             self._step_graph_stream = torch.cuda.Stream(device=self.device)
+            self._step_graph_side = torch.cuda.Stream(device=self.device)
         stream = self._step_graph_stream
         before = kernels.guarded_launch_counts()
         try:
@@ -425,6 +428,7 @@ class StepRunner:
             stream.synchronize()
             after = kernels.guarded_launch_counts()
             graph = torch.cuda.CUDAGraph()
+            ctx.side_stream = self._step_graph_side
             with capture(graph, pool=self._step_graph_pool, stream=stream):
                 logits = self.model.forward(ctx)
         except Exception as failure:                      # noqa: BLE001 (whatever a part or CUDA raises)
@@ -442,6 +446,7 @@ class StepRunner:
             self._step_graph_pool = graph.pool()
         guarded = (after[0] > before[0], after[1] > before[1])      # what one pass of the step launched
         ctx.workspace_of = None       # a replay asks for no scratch; without it the graph does not hold the runner
+        ctx.side_stream = None
         self._step_graphs[ctx.signature] = _StepGraph(graph, ctx.arena, logits, ctx, self._step_count, guarded)
 
     def drop_graphs(self) -> None:

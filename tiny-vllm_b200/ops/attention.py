@@ -18,6 +18,7 @@ max(0, p - window + 1) to p through the block table.
 
 from __future__ import annotations
 
+import contextlib
 import math
 import os
 
@@ -175,6 +176,17 @@ def prefill_tiles(counts, starts=None, *, tensor_memory: bool = False, singles_a
     return big, rest, tuple((first, count) for first, count in runs)
 
 
+@contextlib.contextmanager
+def _branch(side):
+    """Launches inside go to the stream ``side`` (None: nowhere else), behind what was launched so far."""
+    if side is None:
+        yield
+        return
+    side.wait_stream(torch.cuda.current_stream(side.device))
+    with torch.cuda.stream(side):
+        yield
+
+
 def mixer_attention(ctx, mixer, qkv: torch.Tensor, run: int) -> torch.Tensor:
     """From the packed projection ``qkv`` [tokens, (q + 2 kv) * head_dim] of a step to the
     attention output [tokens, q * head_dim]; writes the step's keys and values."""
@@ -217,6 +229,41 @@ def mixer_attention(ctx, mixer, qkv: torch.Tensor, run: int) -> torch.Tensor:
     if (tiled and ctx.tile_row is not None
             and kernels.attention_prefill_supports(mixer.head_dim, mixer.num_heads, mixer.num_kv_heads)):
         out = torch.empty((qkv.shape[0], mixer.num_heads * mixer.head_dim), dtype=qkv.dtype, device=qkv.device)
+        # In a recorded step the single tokens are a branch beside the tiles: the decode kernel is bound by memory and by
+        # the steps inside its clusters, the tile kernels by their longest item (24 single tokens beside 798 of prompts:
+        # 31 us and 17 us a layer in line, 42 us this way: the tiles' CTAs find room as the others leave).  Both read
+        # what the preparing kernel stored and write rows of their own.  (Eager steps are bound by their launches.)
+        side = None
+        if ctx.single_runs and ctx.tile_row.shape[0] + (0 if ctx.tile_tc_row is None else ctx.tile_tc_row.shape[0]) > 0:
+            side = ctx.side_stream
+        with _branch(side):
+            for first, count in ctx.single_runs:
+                # Decoded tokens beside the portions.  Their q is normalised and rotated and their k, v are
+                # in the cache already, so the fused decode kernel runs without its norm, rotation and
+                # cache write: context split over a cluster, keys streamed once per group of q heads.
+                part = slice(first, first + count)
+                splits = fitted_splits(decode_splits(ctx.max_context, count), count, mixer, keys.shape[2], ctx.max_context)
+                if kernels.attention_decode_supports(mixer.head_dim, mixer.num_heads, mixer.num_kv_heads, splits):
+                    kernels.attention_decode(
+                        qkv[part], **heads, positions=ctx.positions[part], token_row=ctx.token_row[part],
+                        slots=None, q_weight=None, k_weight=None, eps=0.0, cos=None, sin=None, key_cache=keys,
+                        value_cache=values, block_tables=ctx.block_tables[group], window=mixer.window,
+                        scale=mixer.scale, splits=splits, max_context=ctx.max_context, out=out[part],
+                        new_in_cache=True,
+                        library_of=None if mixer.q_norm_weight is None else mixer.q_norm_weight.dtype)
+                    continue
+                # chunks for the longest context a request may reach, not for this step's: the count is
+                # then the same for every step with these entry sizes, which a recorded step relies on
+                # (the merge walks only the chunks a row's own position reaches)
+                chunks = choose_split(count, max(ctx.max_context - 1, ctx.max_position))
+                scratch = None
+                if chunks > 0:
+                    scratch = ctx.workspace(kernels.attention_rows_scratch_floats(
+                        count, mixer.num_heads, mixer.head_dim, chunks))
+                kernels.attention_rows(
+                    qkv[part], qkv.shape[1], keys, values, ctx.block_tables[group], ctx.token_row[part],
+                    ctx.positions[part], **heads, window=mixer.window, scale=mixer.scale, out=out[part],
+                    scratch=scratch, max_chunks=chunks)
         if ctx.tile_tc_row is not None and ctx.tile_tc_row.shape[0] > 0:
             # the step's tile lists were cut for the tcgen05 kernel: every mixer of the model takes it
             kernels.attention_prefill_tc(
@@ -226,33 +273,8 @@ def mixer_attention(ctx, mixer, qkv: torch.Tensor, run: int) -> torch.Tensor:
             kernels.attention_prefill(
                 qkv, qkv.shape[1], keys, values, ctx.block_tables[group], ctx.positions, ctx.tile_row,
                 ctx.tile_first, ctx.tile_count, **heads, window=mixer.window, scale=mixer.scale, out=out)
-        for first, count in ctx.single_runs:
-            # Decoded tokens beside the portions.  Their q is normalised and rotated and their k, v are
-            # in the cache already, so the fused decode kernel runs without its norm, rotation and
-            # cache write: context split over a cluster, keys streamed once per group of q heads.
-            part = slice(first, first + count)
-            splits = fitted_splits(decode_splits(ctx.max_context, count), count, mixer, keys.shape[2], ctx.max_context)
-            if kernels.attention_decode_supports(mixer.head_dim, mixer.num_heads, mixer.num_kv_heads, splits):
-                kernels.attention_decode(
-                    qkv[part], **heads, positions=ctx.positions[part], token_row=ctx.token_row[part],
-                    slots=None, q_weight=None, k_weight=None, eps=0.0, cos=None, sin=None, key_cache=keys,
-                    value_cache=values, block_tables=ctx.block_tables[group], window=mixer.window,
-                    scale=mixer.scale, splits=splits, max_context=ctx.max_context, out=out[part],
-                    new_in_cache=True,
-                    library_of=None if mixer.q_norm_weight is None else mixer.q_norm_weight.dtype)
-                continue
-            # chunks for the longest context a request may reach, not for this step's: the count is
-            # then the same for every step with these entry sizes, which a recorded step relies on
-            # (the merge walks only the chunks a row's own position reaches)
-            chunks = choose_split(count, max(ctx.max_context - 1, ctx.max_position))
-            scratch = None
-            if chunks > 0:
-                scratch = ctx.workspace(kernels.attention_rows_scratch_floats(
-                    count, mixer.num_heads, mixer.head_dim, chunks))
-            kernels.attention_rows(
-                qkv[part], qkv.shape[1], keys, values, ctx.block_tables[group], ctx.token_row[part],
-                ctx.positions[part], **heads, window=mixer.window, scale=mixer.scale, out=out[part],
-                scratch=scratch, max_chunks=chunks)
+        if side is not None:
+            torch.cuda.current_stream(side.device).wait_stream(side)
         return out
     scratch = None
     if ctx.split_chunks > 0:
