@@ -15,14 +15,15 @@
 // x is split once, by a small kernel; w on its way into shared memory, by the 16 warps that also add up the sums: its
 // parts are never in memory, and a weight takes no more room than before.  Integer instructions split (the conversion
 // to bfloat16 has a quarter of their rate).  A tile is 128 columns of c by 16 to 128 rows: with two stages of 96 KB no
-// more fits.  A block of 64 k takes 1.4 us at 16 rows and 1.9 at 128, of which the products are 0.6 and 0.9: what bounds
+// more fits.  A block of 64 k takes 1.25 us at 16 rows and 1.65 at 128, of which the products are 0.6 and 0.9: what bounds
 // the kernel is the chain of splitting, handing over, products and sums, two blocks deep, and shared memory, which the
 // products read at nearly its rate.  (Registers decide: at 96 a thread nothing may spill, since 28 KB of L1 are left and
-// the stream of w evicts what is spilled: 2.2 us a block.  Eight warps that split beside eight that add up: 2.0.)
+// the stream of w evicts what is spilled: 2.2 us a block.  Eight warps that split beside eight that add up: 2.0.  Waits by
+// one lane that tells the others: 1.4 and 1.9.)
 //
-// Measured (us, float32 cores / this, weights from memory): 64 rows 4,096 x 1,024 31 / 29, 6,144 x 1,024 43 / 29, 1,024 x
-// 3,072 30 / 31; 301 rows 93 / 33, 127 / 36, 76 / 36; 677 rows 176 / 63, 260 / 70 (121 TFLOP/s), 139 / 46; 2,048 rows
-// 464 / 139, 687 / 196 (132 TFLOP/s), 354 / 122.  Error against 64-bit sums (2-norm) at k = 1,024 / 3,072 / 25,600: 1.10e-7,
+// Measured (us, float32 cores / this, weights from memory): 64 rows 4,096 x 1,024 31 / 25, 6,144 x 1,024 43 / 26, 1,024 x
+// 3,072 30 / 27; 301 rows 93 / 30, 127 / 32, 76 / 32; 677 rows 176 / 56, 260 / 63 (136 TFLOP/s), 139 / 40; 2,048 rows
+// 464 / 121, 687 / 176 (147 TFLOP/s), 354 / 104.  Error against 64-bit sums (2-norm) at k = 1,024 / 3,072 / 25,600: 1.10e-7,
 // 1.16e-7, 1.46e-7 (float32 cores 1.55e-7, 1.60e-7, 2.02e-7); of that 6e-8 is what the tensor cores cut off.
 #include <algorithm>
 
@@ -150,14 +151,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_base_slot;
-    // waits of a whole warp: one lane waits with the limit and tells the others
+    // waits of a whole warp
     auto warp_wait = [&](uint32_t bar, uint32_t parity, int code) {
-        int ready = lane == 0 ? (int)mbar_wait(bar, parity, abort_flag, status, code) : 1;
-        ready = __shfl_sync(0xffffffffu, ready, 0);
-        if (ready)
-            for (int tries = 0; tries < 1024 && !mbar_try(bar, parity); ++tries) {}
-        __syncwarp();
-        return ready != 0;
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code)) != 0;
     };
 
     if (warp < WORK_WARPS) {
@@ -338,7 +334,7 @@ Plan plan_of(int m, int n, int k, int sms) {
     double least = 0.0;
     for (int tiles = fewest; tiles <= fewest + 4 && tiles <= (m + 15) / 16; ++tiles) {
         const int nx = ((m + tiles - 1) / tiles + 15) / 16 * 16, tiles_x = (m + nx - 1) / nx;
-        const double block_us = 1.42 + 0.0035 * nx;
+        const double block_us = 1.2 + 0.0035 * nx;
         for (int per = best.groups; per >= 1; --per) {
             const int splits = (best.groups + per - 1) / per;
             if (splits > 1 && ((long long)best.groups * m * n > SCRATCH_FLOATS || splits > 65535)) break;

@@ -32,8 +32,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, *, out_dtype: torch.dtype | No
     return gemm.linear_bf16(x, weight, out_dtype=out_dtype, out=out)
 
 
-# Rows up to which a float32 product stays on the float32 cores: the tensor-core kernel takes 28 to 31 us for a layer's
-# products at any number of rows up to 128 (a CTA walks 1,024 k in 16 steps of 1.4 us), the float32 cores 16 to 24 us
+# Rows up to which a float32 product stays on the float32 cores: the tensor-core kernel takes 25 to 28 us for a layer's
+# products at any number of rows up to 128 (a CTA walks 1,024 k in 16 steps of 1.2 us), the float32 cores 16 to 24 us
 # for 32 rows, 29 to 42 us for 48.
 F32_CORE_ROWS = 32
 
