@@ -43,3 +43,13 @@ def test_weights_and_products_of_the_launch_before_are_awaited(width):
         kernels.rms_norm(x, weight, 1e-6, out=made)
         got = kernels.gemm_nt_simt(rows, made[2900:])                # a weight that the launch before writes
         assert torch.equal(got, kernels.gemm_nt_simt(rows, made[2900:].clone())), turn
+
+
+@pytest.mark.parametrize("inter", [1, 6, 8, 1020, 1028, 3072])
+def test_silu_times_up(inter):
+    generator = torch.Generator(device="cuda").manual_seed(inter)
+    packed = torch.randn(5, 2 * inter, generator=generator, device="cuda") * 4
+    gate, up = packed.double().split(inter, dim=1)
+    want = gate / (1 + torch.exp(-gate)) * up
+    for rows in (packed, torch.empty(10 * inter + 1, device="cuda")[1:].view(5, 2 * inter).copy_(packed)):   # (off the boundary)
+        assert ((kernels.silu_mul(rows).double() - want).abs() <= 8 * 2.0 ** -24 * want.abs() + 1e-37).all()

@@ -102,8 +102,9 @@ __device__ float plain_sum(const float* x, const float* w, int k_from, int k_to)
 
 // A row of x a block: its three parts, [3][m][kp] with zeros from k on, and whether it holds a value that has none.
 __global__ void __launch_bounds__(128)
-split_rows_kernel(const float* __restrict__ a, int64_t lda, uint2* parts, int* wild_x, int m, int k, int kp) {
+split_rows_kernel(const float* a, int64_t lda, uint2* parts, int* wild_x, int m, int k, int kp) {
     pdl_launch_dependents();
+    pdl_wait();
     const int row = blockIdx.x;
     float2 wild = make_float2(0.0f, 0.0f);
     for (int at = threadIdx.x * 4; at < kp; at += 128 * 4) {
@@ -121,8 +122,7 @@ split_rows_kernel(const float* __restrict__ a, int64_t lda, uint2* parts, int* w
 // whose sums meet in c; else group g goes to partial[g][m][n].  map_x: the parts of x.
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x, const float* a, int64_t lda,
-                   const float* __restrict__ w, int64_t ldw, float* c, int64_t ldc, float* partial, int groups_per, int m, int n,
-                   int k, int nx) {
+                   const float* w, int64_t ldw, float* c, int64_t ldc, float* partial, int groups_per, int m, int n, int k, int nx) {
     extern __shared__ uint8_t raw_shared[];
     const uint32_t base = (smem_address(raw_shared) + 1023u) & ~1023u;
     uint8_t* aligned = raw_shared + (base - smem_address(raw_shared));
@@ -311,14 +311,23 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
     }
 }
 
-// c = the sum of the groups' partial products, in ascending order
+// c = the sum of the groups' partial products, in ascending order; VEC neighbouring columns a thread.
+template <int VEC>
 __global__ void __launch_bounds__(256)
 fold_groups_kernel(const float* __restrict__ partial, int groups, float* __restrict__ c, int64_t ldc, int m, int n) {
-    const int64_t size = (int64_t)m * n;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += (int64_t)gridDim.x * blockDim.x) {
-        float total = partial[i];
-        for (int g = 1; g < groups; ++g) total = __fadd_rn(total, partial[g * size + i]);
-        c[(i / n) * ldc + i % n] = total;
+    const int words = n / VEC;
+    const int64_t size = (int64_t)m * n, total = (int64_t)m * words;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t row = total <= 0x7fffffff ? (uint32_t)i / (uint32_t)words : i / words;
+        const int64_t at = (i - row * words) * VEC;
+        float sum[VEC], more[VEC];
+        load_values<VEC>(partial + row * n + at, sum);
+        for (int g = 1; g < groups; ++g) {
+            load_values<VEC>(partial + g * size + row * n + at, more);
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) sum[j] = __fadd_rn(sum[j], more[j]);
+        }
+        store_values<VEC>(c + row * ldc + at, sum);
     }
 }
 
@@ -381,9 +390,11 @@ extern "C" int tvb_gemm_f32_tc_launches(int m, int n, int k) {
 }
 
 // c[m, n] = a . w^T; rows of a and w on 16-byte boundaries.  scratch: tvb_gemm_f32_tc_scratch_bytes, on a 128-byte
-// boundary.  nx, splits: 0, or force the rows of a tile and the pieces of k.
+// boundary.  nx, splits: 0, or force the rows of a tile and the pieces of k.  w_constant: no launch that may still run
+// writes w.
 extern "C" int tvb_gemm_f32_tc(const float* a, long long lda, const float* w, long long ldw, float* c, long long ldc, int m,
-                               int n, int k, uint8_t* scratch, int nx, int splits, int pdl, void* stream) {
+                               int n, int k, uint8_t* scratch, int nx, int splits, int pdl, int w_constant,
+                               void* stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0 || k % 4 || lda % 4 || ldw % 4 || !scratch ||
         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) || (reinterpret_cast<uintptr_t>(scratch) & 127))
@@ -410,16 +421,20 @@ extern "C" int tvb_gemm_f32_tc(const float* a, long long lda, const float* w, lo
     cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_BYTES);
     if (e != cudaSuccess) return (int)e;
     cudaStream_t s = (cudaStream_t)stream;
-    split_rows_kernel<<<m, 128, 0, s>>>(a, lda, reinterpret_cast<uint2*>(parts), wild_x, m, k, (int)kp);
-    e = cudaGetLastError();
+    // The product's kernel reads w without waiting: the kernel that splits x, which it follows, starts behind all launches
+    // before, unless none of those that may still run writes w.
+    TvbLaunch split(dim3(m), dim3(128), 0, s, pdl && w_constant);
+    e = cudaLaunchKernelEx(&split.config, split_rows_kernel, a, (int64_t)lda, reinterpret_cast<uint2*>(parts), wild_x, m, k, (int)kp);
     if (e != cudaSuccess) return (int)e;
     TvbLaunch launch(dim3((n + BW - 1) / BW, plan.tiles_x, plan.splits), dim3(THREADS), SHARED_BYTES, s, pdl);
     e = cudaLaunchKernelEx(&launch.config, gemm_f32_tc_kernel, map_x, (const int*)wild_x, a, (int64_t)lda, w, (int64_t)ldw, c,
                            (int64_t)ldc, partial, plan.groups_per, m, n, k, plan.nx);
     if (e != cudaSuccess) return (int)e;
     if (plan.splits > 1) {
-        const int blocks = (int)std::min<long long>(((long long)m * n + 255) / 256, 8LL * sms);
-        fold_groups_kernel<<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n);
+        const bool by_four = n % 4 == 0 && ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
+        const int blocks = (int)std::min<long long>(((long long)m * n / (by_four ? 4 : 1) + 255) / 256, 8LL * sms);
+        if (by_four) fold_groups_kernel<4><<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n);
+        else fold_groups_kernel<1><<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n);
     }
     return tvb_last_error();
 }

@@ -59,7 +59,7 @@ def _pdl(kind: str) -> int:
 
 
 # Rows up to which the elementwise kernels between float32 products are launched programmatically: their grids are small
-# then and leave the kernel before its SMs (677 rows of SiLU * up: 9.3 us with, 6.8 without).
+# then and leave the kernel before its SMs (677 rows of SiLU * up at a value a thread: 9.3 us with, 6.8 without).
 PDL_FEW_ROWS = 32
 
 
@@ -1903,9 +1903,11 @@ def gemm_f32_tc_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
             and a.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
-def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, *,
+                weight_constant: bool = False) -> torch.Tensor:
     """a [m, k] . w [n, k]^T of float32 operands on the tensor cores, each operand as three bfloat16 whose products are
-    added up to float32 sums; the order of a sum over k depends on k alone."""
+    added up to float32 sums; the order of a sum over k depends on k alone.  ``weight_constant``: no kernel that may still
+    run writes w, which is then read before the kernel before has ended."""
     _need_cuda(a, w)
     if not gemm_f32_tc_takes(a, w):
         raise KernelError("gemm_f32_tc wants float32 a [m, k] and w [n, k] with contiguous, 16-byte aligned rows, "
@@ -1924,10 +1926,10 @@ def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = Non
                           device=a.device)
     fn = _fn("gemm_f32_tc", "tvb_gemm_f32_tc",
              [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_int,
-              c_int, c_int, c_void_p])
+              c_int, c_int, c_int, c_void_p])
     global _gemm_tc_unchecked, _gemm_f32_tc_used
     _check(fn(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), m, n, k,
-              scratch.data_ptr(), 0, 0, _pdl("gemm"), _stream()), "gemm_f32_tc",
+              scratch.data_ptr(), 0, 0, _pdl("gemm"), 1 if weight_constant else 0, _stream()), "gemm_f32_tc",
            _fn("gemm_f32_tc", "tvb_gemm_f32_tc_launches", sizes)(m, n, k))
     _gemm_tc_unchecked = _gemm_f32_tc_used = True
     _guarded_counts[0] += 1

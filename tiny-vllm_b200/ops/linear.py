@@ -40,7 +40,7 @@ F32_CORE_ROWS = 32
 
 def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None) -> torch.Tensor:
     if x.shape[0] > F32_CORE_ROWS and kernels.gemm_f32_tc_takes(x, weight):
-        return kernels.gemm_f32_tc(x, weight, out=out)
+        return kernels.gemm_f32_tc(x, weight, out=out, weight_constant=True)
     return kernels.gemm_nt_simt(x, weight, out=out, weight_constant=True)
 
 
