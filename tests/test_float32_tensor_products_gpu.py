@@ -75,3 +75,13 @@ def test_which_kernel_takes_a_product():
     assert torch.equal(linear(off, w), kernels.gemm_nt_simt(off, w))
     odd = a[:, :127].contiguous()
     assert torch.equal(linear(odd, w[:, :127].contiguous()), kernels.gemm_nt_simt(odd, w[:, :127].contiguous()))
+
+
+def test_products_in_ranges_of_rows():
+    """More rows than 64 MiB of parts hold: the ranges' sums are those of a product of their own."""
+    generator = torch.Generator(device=DEV).manual_seed(6)
+    a = torch.randn(1100, 25600, generator=generator, device=DEV)
+    w = torch.randn(40, 25600, generator=generator, device=DEV)
+    whole = kernels.gemm_f32_tc(a, w)
+    assert torch.equal(whole[1000:], kernels.gemm_f32_tc(a[1000:], w)) and torch.equal(whole[:50], kernels.gemm_f32_tc(a[:50], w))
+    assert ((whole.double() - a.double() @ w.double().T).abs() <= bound(a, w)).all()

@@ -26,6 +26,7 @@
 // 464 / 121, 687 / 176 (147 TFLOP/s), 354 / 104.  Error against 64-bit sums (2-norm) at k = 1,024 / 3,072 / 25,600: 1.10e-7,
 // 1.16e-7, 1.46e-7 (float32 cores 1.55e-7, 1.60e-7, 2.02e-7); of that 6e-8 is what the tensor cores cut off.
 #include <algorithm>
+#include <initializer_list>
 
 #include "tc5.cuh"
 
@@ -359,8 +360,18 @@ Plan plan_of(int m, int n, int k, int sms) {
     return best;
 }
 
-// Scratch of a product: partial sums, the parts of x, and a word a row of x.
+// Scratch of a product: partial sums, the parts of x, and a word a row of x.  Partial sums take up to 64 MiB and so do the
+// parts (128 rows, where those take more): a product of more rows runs a range of rows at a time.
 long long padded_k(int k) { return (k + BK - 1) / BK * BK; }
+int range_rows(int m, int k) {
+    const long long fit = std::max(128LL, SCRATCH_FLOATS * 4 / (6 * padded_k(k)) / 128 * 128);
+    const long long ranges = (m + fit - 1) / fit;
+    return ranges <= 1 ? m : (int)(((m + ranges - 1) / ranges + 127) / 128 * 128);
+}
+int plan_sms() {
+    const int sms = tvb_sm_count();
+    return sms > 0 ? sms : 148;                       // (asked for sizes without a device)
+}
 long long sum_bytes(const Plan& plan, int m, int n) {
     return plan.splits > 1 ? ((long long)plan.groups * m * n * 4 + 127) / 128 * 128 : 0;
 }
@@ -377,35 +388,24 @@ extern "C" int tvb_gemm_f32_tc_status() {
 }
 
 extern "C" long long tvb_gemm_f32_tc_scratch_bytes(int m, int n, int k) {
-    const int sms = tvb_sm_count();
-    if (m <= 0 || n <= 0 || k <= 0 || sms <= 0) return 0;
-    return sum_bytes(plan_of(m, n, k, sms), m, n) + 3 * m * padded_k(k) * 2 + 4ll * m;
+    if (m <= 0 || n <= 0 || k <= 0) return 0;
+    const int rows = range_rows(m, k), last = m - (m - 1) / rows * rows;
+    long long most = 0;
+    for (int of : {rows, last})
+        most = std::max(most, sum_bytes(plan_of(of, n, k, plan_sms()), of, n) + 3 * of * padded_k(k) * 2 + 4ll * of);
+    return most;
 }
 
 // kernels that a product launches
 extern "C" int tvb_gemm_f32_tc_launches(int m, int n, int k) {
-    const int sms = tvb_sm_count();
-    if (m <= 0 || n <= 0 || k <= 0 || sms <= 0) return 0;
-    return plan_of(m, n, k, sms).splits > 1 ? 3 : 2;
+    if (m <= 0 || n <= 0 || k <= 0) return 0;
+    const int rows = range_rows(m, k), last = m - (m - 1) / rows * rows;
+    return (m - 1) / rows * (plan_of(rows, n, k, plan_sms()).splits > 1 ? 3 : 2) + (plan_of(last, n, k, plan_sms()).splits > 1 ? 3 : 2);
 }
 
-// c[m, n] = a . w^T; rows of a and w on 16-byte boundaries.  scratch: tvb_gemm_f32_tc_scratch_bytes, on a 128-byte
-// boundary.  nx, splits: 0, or force the rows of a tile and the pieces of k.  w_constant: no launch that may still run
-// writes w.
-extern "C" int tvb_gemm_f32_tc(const float* a, long long lda, const float* w, long long ldw, float* c, long long ldc, int m,
-                               int n, int k, uint8_t* scratch, int nx, int splits, int pdl, int w_constant,
-                               void* stream) {
-    if (m <= 0 || n <= 0) return 0;
-    if (k <= 0 || k % 4 || lda % 4 || ldw % 4 || !scratch ||
-        ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) || (reinterpret_cast<uintptr_t>(scratch) & 127))
-        return TVB_BAD_ARGUMENT;
-    const int sms = tvb_sm_count();
-    if (sms <= 0) return (int)cudaErrorInvalidDevice;
-    Plan plan = plan_of(m, n, k, sms);
-    if (nx > 0) {
-        plan.nx = nx; plan.tiles_x = (m + nx - 1) / nx;
-        plan.groups_per = (plan.groups + splits - 1) / splits; plan.splits = (plan.groups + plan.groups_per - 1) / plan.groups_per;
-    }
+static int launch_range(const float* a, long long lda, const float* w, long long ldw, float* c, long long ldc, int m, int n, int k,
+                        uint8_t* scratch, int sms, int pdl, int w_constant, cudaStream_t s) {
+    const Plan plan = plan_of(m, n, k, sms);
     if (plan.tiles_x > 65535) return TVB_BAD_ARGUMENT;
     float* partial = plan.splits > 1 ? reinterpret_cast<float*>(scratch) : nullptr;
     uint8_t* parts = scratch + sum_bytes(plan, m, n);
@@ -420,7 +420,6 @@ extern "C" int tvb_gemm_f32_tc(const float* a, long long lda, const float* w, lo
     }
     cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_BYTES);
     if (e != cudaSuccess) return (int)e;
-    cudaStream_t s = (cudaStream_t)stream;
     // The product's kernel reads w without waiting: the kernel that splits x, which it follows, starts behind all launches
     // before, unless none of those that may still run writes w.
     TvbLaunch split(dim3(m), dim3(128), 0, s, pdl && w_constant);
@@ -437,4 +436,23 @@ extern "C" int tvb_gemm_f32_tc(const float* a, long long lda, const float* w, lo
         else fold_groups_kernel<1><<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n);
     }
     return tvb_last_error();
+}
+
+// c[m, n] = a . w^T; rows of a and w on 16-byte boundaries.  scratch: tvb_gemm_f32_tc_scratch_bytes, on a 128-byte
+// boundary.  w_constant: no launch that may still run writes w.
+extern "C" int tvb_gemm_f32_tc(const float* a, long long lda, const float* w, long long ldw, float* c, long long ldc, int m,
+                               int n, int k, uint8_t* scratch, int pdl, int w_constant, void* stream) {
+    if (m <= 0 || n <= 0) return 0;
+    if (k <= 0 || k % 4 || lda % 4 || ldw % 4 || !scratch ||
+        ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) || (reinterpret_cast<uintptr_t>(scratch) & 127))
+        return TVB_BAD_ARGUMENT;
+    const int sms = tvb_sm_count();
+    if (sms <= 0) return (int)cudaErrorInvalidDevice;
+    const int rows = range_rows(m, k);
+    for (int at = 0; at < m; at += rows) {
+        const int status = launch_range(a + at * lda, lda, w, ldw, c + at * ldc, ldc, std::min(rows, m - at), n, k, scratch, sms,
+                                        pdl, w_constant, (cudaStream_t)stream);
+        if (status != 0) return status;
+    }
+    return 0;
 }

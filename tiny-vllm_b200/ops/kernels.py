@@ -1920,23 +1920,27 @@ def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = Non
         raise KernelError("gemm_f32_tc: out must be float32 [m, n] with contiguous rows")
     if m == 0 or n == 0:
         return out
-    sizes = [c_int, c_int, c_int]
     # the parts of a, and partial sums where k is cut
-    scratch = torch.empty(_fn("gemm_f32_tc", "tvb_gemm_f32_tc_scratch_bytes", sizes, c_longlong)(m, n, k), dtype=torch.uint8,
-                          device=a.device)
+    scratch = torch.empty(gemm_f32_tc_scratch_bytes(m, n, k), dtype=torch.uint8, device=a.device)
     fn = _fn("gemm_f32_tc", "tvb_gemm_f32_tc",
              [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_int,
-              c_int, c_int, c_int, c_void_p])
+              c_int, c_void_p])
     global _gemm_tc_unchecked, _gemm_f32_tc_used
     _check(fn(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), m, n, k,
-              scratch.data_ptr(), 0, 0, _pdl("gemm"), 1 if weight_constant else 0, _stream()), "gemm_f32_tc",
-           _fn("gemm_f32_tc", "tvb_gemm_f32_tc_launches", sizes)(m, n, k))
+              scratch.data_ptr(), _pdl("gemm"), 1 if weight_constant else 0, _stream()), "gemm_f32_tc",
+           _fn("gemm_f32_tc", "tvb_gemm_f32_tc_launches", [c_int, c_int, c_int])(m, n, k))
     _gemm_tc_unchecked = _gemm_f32_tc_used = True
     _guarded_counts[0] += 1
     return out
 
 
 _gemm_f32_tc_used = False
+
+
+def gemm_f32_tc_scratch_bytes(m: int, n: int, k: int) -> int:
+    """Scratch of a product on the tensor cores: up to 64 MiB of partial sums and 64 MiB of parts of a (128 rows, where those
+    take more)."""
+    return _fn("gemm_f32_tc", "tvb_gemm_f32_tc_scratch_bytes", [c_int, c_int, c_int], c_longlong)(m, n, k)
 
 
 def gemm_f32_tc_status() -> int:
