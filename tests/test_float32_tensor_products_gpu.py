@@ -1,5 +1,6 @@
 """Products of float32 operands on the tensor cores: against 64 bits at the edges of tiles, blocks and groups of k, values
-that have no three bfloat16 parts, and that a row's sum does not depend on the other rows."""
+that have no three bfloat16 parts, products at the end of the float32 range, and that a row's sum does not depend on the other
+rows."""
 
 import pytest
 import torch
@@ -55,6 +56,60 @@ def test_values_without_three_parts(value, k):
         same = torch.isfinite(at)
         assert (at[same].abs() <= 1e-5 * k * max(1.0, 1e36 if abs(value) < float("inf") else 1.0)).all()
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+
+
+def same_where_not_finite(got, want):
+    return torch.equal(got.isnan(), want.isnan()) and torch.equal(got == float("inf"), want == float("inf")) and torch.equal(
+        got == float("-inf"), want == float("-inf"))
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 130, 64), (150, 140, 1028), (150, 140, 2048), (2500, 1500, 2052)])
+def test_products_beyond_float32_are_summed_as_the_float32_cores_do(m, n, k):
+    """Finite operands whose products, or parts' products, leave float32: whole, cut and added up from partial sums."""
+    generator = torch.Generator(device=DEV).manual_seed(k)
+    a, w = torch.randn(m, k, generator=generator, device=DEV), torch.randn(n, k, generator=generator, device=DEV)
+    a, w = a + a.sign(), w + w.sign()                       # none near zero: every product below is beyond float32
+    for scale in (1e20, 1e21, 3e37):
+        got, want = kernels.gemm_f32_tc(a * scale, w * scale), kernels.gemm_nt_simt(a * scale, w * scale)
+        assert same_where_not_finite(got, want) and not want.isfinite().any(), scale
+    # a row and a column of them, the rest as ever
+    clean, some = kernels.gemm_f32_tc(a, w), a.clone()
+    some[m - 3] *= 1e38
+    got, want = kernels.gemm_f32_tc(some, w), kernels.gemm_nt_simt(some, w)
+    kept = torch.arange(m, device=DEV) != m - 3
+    assert torch.equal(got[kept], clean[kept]) and same_where_not_finite(got, want)
+    # a NaN in a row, infinities of either sign in another and in a column
+    some = a.clone()
+    some[3, 7], some[20, k - 1], some[20, 0] = float("nan"), float("inf"), float("-inf")
+    wide = w.clone()
+    wide[11, 5] = float("inf")
+    got, want = kernels.gemm_f32_tc(some, wide), kernels.gemm_nt_simt(some, wide)
+    assert same_where_not_finite(got, want) and got[3].isnan().all()
+    kept[m - 3], kept[3], kept[20] = True, False, False
+    others = torch.arange(n, device=DEV) != 11
+    assert torch.equal(got[kept][:, others], clean[kept][:, others])
+
+
+@pytest.mark.parametrize("k", [64, 1024, 2048])
+def test_products_just_inside_float32(k):
+    """u * v up to the largest float32: the first parts round up and their product is beyond it.  Alone, and two that cancel."""
+    generator = torch.Generator(device=DEV).manual_seed(k + 1)
+    largest = torch.finfo(torch.float32).max
+    u = (1.0 + torch.rand(150, generator=generator, device=DEV, dtype=torch.float64)).float()
+    v = (1.06 - 0.08 * torch.rand(140, generator=generator, device=DEV, dtype=torch.float64)).float()
+    u[:75] = 2.0 - 0.008 * (u[:75] - 1.0)
+    a, w = torch.zeros(150, k, device=DEV), torch.zeros(140, k, device=DEV)
+    a[:, 5], w[:, 5] = u * 2.0 ** 63, v * 2.0 ** 64          # products from 2^126 to beyond the largest float32, many near it
+    want = a[:, 5:6].double() @ w[:, 5:6].double().T
+    inside = want.abs() <= largest
+    near = inside & (want.abs() > 0.98 * largest)
+    assert near.sum() > 100 and not inside.all()
+    got = kernels.gemm_f32_tc(a, w)
+    assert got[inside].isfinite().all() and got[~inside & (want > 1.0001 * largest)].isinf().all()
+    assert ((got.double() - want).abs()[inside] <= bound(a, w)[inside]).all()
+    a[:, k - 2], w[:, k - 2] = a[:, 5], -w[:, 5]             # the same once more with the other sign, far along k
+    got = kernels.gemm_f32_tc(a, w)
+    assert (got[inside].abs() <= bound(a, w)[inside]).all() and torch.equal(got[near], kernels.gemm_nt_simt(a, w)[near])
 
 
 @pytest.mark.parametrize("scale", [1e-30, 1e-18, 1e18, 1e30])

@@ -9,8 +9,10 @@
 // tensor cores cut off what does not fit instead of rounding it, which over all of k would shrink the sums.
 //
 // The sum of an output element has one order whatever m is: blocks of 64 k ascending inside a group of 1,024, the groups
-// ascending.  Operands with infinities, NaN or values that round to infinity in bfloat16 have no such three parts: the
-// rows and columns that hold one are summed again by the float32 cores from the operands themselves.
+// ascending.  Infinities, NaN and values that round to infinity in bfloat16 have no such three parts, and the product of two
+// parts can be beyond float32 where x w is not (x1 and w1 round up) or is with one sign (x1 w2 has the other: NaN).  All of it
+// ends in a sum that is not finite: such an element is summed again by the float32 cores from the operands themselves, and has
+// their bits.
 //
 // x is split once, by a small kernel; w on its way into shared memory, by the 16 warps that also add up the sums: its
 // parts are never in memory, and a weight takes no more room than before.  Integer instructions split (the conversion
@@ -46,7 +48,7 @@ constexpr int STAGES = 2;
 constexpr int PART_BYTES = 128 * BK * 2;                 // one of the three parts of 128 rows
 constexpr int STAGE_BYTES = 6 * PART_BYTES;              // of w, then of x
 constexpr int BARRIERS = 4;
-constexpr int SHARED_BYTES = STAGES * STAGE_BYTES + BARRIERS * 8 + 16 + 256 + 1024;
+constexpr int SHARED_BYTES = STAGES * STAGE_BYTES + BARRIERS * 8 + 16 + 1024;
 constexpr uint32_t TMEM_COLS = 2 * MAX_X;
 constexpr int ROWS_A_PASS = WORKERS / (BK / 4);          // 32: a thread takes 4 k of every 32nd row of w
 constexpr int PASSES = 128 / ROWS_A_PASS;
@@ -62,8 +64,8 @@ __device__ __forceinline__ float2 fma_two(float2 a, float2 b, float2 c) {
     return r.f;
 }
 
-// Four float32 as three times four bfloat16.  `wild` becomes NaN if a value has no such parts.
-__device__ __forceinline__ void split_four(const float4& x, uint2* part, float2& wild) {
+// Four float32 as three times four bfloat16.
+__device__ __forceinline__ void split_four(const float4& x, uint2* part) {
     float2 rest[2] = {make_float2(x.x, x.y), make_float2(x.z, x.w)};
     uint32_t* words = reinterpret_cast<uint32_t*>(part);
 #pragma unroll
@@ -77,7 +79,6 @@ __device__ __forceinline__ void split_four(const float4& x, uint2* part, float2&
             rest[j] = fma_two(make_float2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)),
                               make_float2(-1.0f, -1.0f), rest[j]);           // exact
         }
-        wild = fma_two(rest[j], make_float2(0.0f, 0.0f), wild);
     }
 }
 
@@ -94,35 +95,101 @@ __device__ __forceinline__ bool elect_lane() {
     return elected != 0;
 }
 
-// The sum over [k_from, k_to) by the float32 cores, for operands that cannot be split.
-__device__ float plain_sum(const float* x, const float* w, int k_from, int k_to) {
-    float sum = 0.0f;
-    for (int at = k_from; at < k_to; ++at) sum = __fmaf_rn(x[at], w[at], sum);
-    return sum;
+constexpr int AGAIN_K = 32, AGAIN_STRIDE = AGAIN_K + 4;  // k of a step, floats from row to row in shared memory (the banks)
+constexpr int AGAIN_ROWS = 4;                           // rows of x at a time
+template <int ROWS> constexpr int AGAIN_FLOATS = (32 + ROWS) * AGAIN_STRIDE;            // shared memory of a warp
+static_assert(WORK_WARPS * AGAIN_FLOATS<AGAIN_ROWS> * 4 <= STAGES * STAGE_BYTES, "it lies where the stages were");
+
+// Elements of c that are not finite, of ROWS rows from `row` on and a column a lane (bit i of `again`: row + i), are summed again
+// from the operands by the float32 cores, in the order of gemm_simt.cu (segments of 128 k, a chain over the even and one over the
+// odd k of each; four segments a group, the groups ascending): those with infinities, and those where a part's product or a sum
+// of products is beyond float32 although theirs need not be.  A row of x with a NaN has nothing but NaN already.
+// What is left is finite again, or NaN from the next norm on, so that this runs rarely: 677 x 1,024 x 6,144 takes 61 us, with an
+// infinity in one row 87, all NaN 74, all infinities 920 (the float32 cores 261); 677 x 3,072 x 1,024, added up from partial
+// sums, 37, 460, 45 and 1,390 (139).
+template <int ROWS>
+__device__ __noinline__ void sum_again(unsigned again, int row, int col, const float* a, int64_t lda, const float* w, int64_t ldw,
+                                       float* c, int64_t ldc, int m, int k, const int* nan_rows, float* tile) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+        if (row + i < m && nan_rows[row + i]) again &= ~(1u << i);
+    const unsigned cols = __ballot_sync(0xffffffffu, again != 0);
+    if (cols == 0) return;
+    float4 held[8];                                                  // of w: 4 k of every fourth column
+    float held_x[ROWS];
+    auto load = [&](int at) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int of = i * 4 + lane / 8, of_col = __shfl_sync(0xffffffffu, col, of), from = at + (lane & 7) * 4;
+            held[i] = (cols >> of & 1) && from < k ? *reinterpret_cast<const float4*>(w + (int64_t)of_col * ldw + from)
+                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) held_x[i] = row + i < m && at + lane < k ? a[(int64_t)(row + i) * lda + at + lane] : 0.0f;
+    };
+    float even[ROWS], odd[ROWS], group[ROWS], total[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) even[i] = odd[i] = group[i] = total[i] = 0.0f;
+    load(0);
+    for (int at = 0; at < k; at += AGAIN_K) {
+        __syncwarp();                                                // (what is in the tile has been read)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<float4*>(tile + (i * 4 + lane / 8) * AGAIN_STRIDE + (lane & 7) * 4) = held[i];
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) tile[(32 + i) * AGAIN_STRIDE + lane] = held_x[i];
+        __syncwarp();
+        if (at + AGAIN_K < k) load(at + AGAIN_K);
+#pragma unroll
+        for (int q = 0; q < AGAIN_K; q += 4) {                       // (zeros behind k)
+            const float4 wv = *reinterpret_cast<const float4*>(tile + lane * AGAIN_STRIDE + q);
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                const float4 xv = *reinterpret_cast<const float4*>(tile + (32 + i) * AGAIN_STRIDE + q);
+                even[i] = __fmaf_rn(xv.z, wv.z, __fmaf_rn(xv.x, wv.x, even[i]));
+                odd[i] = __fmaf_rn(xv.w, wv.w, __fmaf_rn(xv.y, wv.y, odd[i]));
+            }
+        }
+        const int segment = at / 128;
+        const bool last = at + AGAIN_K >= k;
+        if ((at + AGAIN_K) % 128 != 0 && !last) continue;
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            const float sum = __fadd_rn(even[i], odd[i]);
+            group[i] = segment % 4 == 0 ? sum : __fadd_rn(group[i], sum);
+            if (segment % 4 == 3 || last) total[i] = segment < 4 ? group[i] : __fadd_rn(total[i], group[i]);
+            even[i] = odd[i] = 0.0f;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+        if (again >> i & 1) c[(int64_t)(row + i) * ldc + col] = total[i];
 }
 
-// A row of x a block: its three parts, [3][m][kp] with zeros from k on, and whether it holds a value that has none.
+// A row of x a block: its three parts, [3][m][kp] with zeros from k on, and whether it holds a NaN.
 __global__ void __launch_bounds__(128)
-split_rows_kernel(const float* a, int64_t lda, uint2* parts, int* wild_x, int m, int k, int kp) {
+split_rows_kernel(const float* a, int64_t lda, uint2* parts, int* nan_rows, int m, int k, int kp) {
     pdl_launch_dependents();
     pdl_wait();
     const int row = blockIdx.x;
-    float2 wild = make_float2(0.0f, 0.0f);
+    bool nan = false;
     for (int at = threadIdx.x * 4; at < kp; at += 128 * 4) {
+        const float4 x = at < k ? *reinterpret_cast<const float4*>(a + (int64_t)row * lda + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+        nan |= x.x != x.x || x.y != x.y || x.z != x.z || x.w != x.w;
         uint2 part[3];
-        split_four(at < k ? *reinterpret_cast<const float4*>(a + (int64_t)row * lda + at) : make_float4(0.f, 0.f, 0.f, 0.f), part,
-                   wild);
+        split_four(x, part);
 #pragma unroll
         for (int i = 0; i < 3; ++i) parts[((int64_t)(i * m + row) * kp + at) / 4] = part[i];
     }
-    const int any = __syncthreads_or(wild.x != 0.0f || wild.y != 0.0f);                 // (NaN)
-    if (threadIdx.x == 0) wild_x[row] = any;
+    const int any = __syncthreads_or(nan);
+    if (threadIdx.x == 0) nan_rows[row] = any;
 }
 
 // One CTA: a tile of up to 128 columns of c and `nx` rows, over groups [z * groups_per, ...) of k.  partial == nullptr: all groups,
 // whose sums meet in c; else group g goes to partial[g][m][n].  map_x: the parts of x.
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x, const float* a, int64_t lda,
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* nan_rows, const float* a, int64_t lda,
                    const float* w, int64_t ldw, float* c, int64_t ldc, float* partial, int groups_per, int m, int n, int k, int nx) {
     extern __shared__ uint8_t raw_shared[];
     const uint32_t base = (smem_address(raw_shared) + 1023u) & ~1023u;
@@ -132,7 +199,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
     auto done_bar = [&](int s) { return bars + 8u * (STAGES + s); };
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(aligned + STAGES * STAGE_BYTES + BARRIERS * 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
-    volatile uint8_t* wild_rows = reinterpret_cast<volatile uint8_t*>(tmem_base_slot + 4);      // [128] of w, [128] of x
+    volatile int* not_finite = abort_flag + 1;          // whether an element of c is not
     int* status = &tvb_gemm_f32_tc_status_word;
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -142,11 +209,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), WORK_WARPS + 1); mbar_init(done_bar(s), 1); }
-        *abort_flag = 0;
+        *abort_flag = *not_finite = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         prefetch_tensormap(&map_x);
     }
-    if (threadIdx.x < BW) wild_rows[threadIdx.x] = 0;
     if (warp == 0) tmem_alloc(smem_address(tmem_base_slot), TMEM_COLS);
     tc_fence_before_sync();
     __syncthreads();
@@ -166,7 +232,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
         const float* w_from = w + (int64_t)(col0 + r0) * ldw + k_from + chunk * 4;
         const uint32_t w_at = base + (uint32_t)(r0 * 128 + (((chunk >> 1) ^ (r0 & 7)) << 4) + (chunk & 1) * 8);   // (32 rows: the same)
         float4 held[PASSES];
-        float2 wild = make_float2(0.0f, 0.0f);
         auto load = [&](int pass, int block) {
             const bool in = col0 + r0 + pass * ROWS_A_PASS < n && k_from + block * BK + chunk * 4 < k_to;
             held[pass] = in ? *reinterpret_cast<const float4*>(w_from + (int64_t)(pass * ROWS_A_PASS) * ldw + block * BK)
@@ -185,7 +250,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
 #pragma unroll
                 for (int pass = 0; pass < PASSES; ++pass) {
                     uint2 part[3];
-                    split_four(held[pass], part, wild);
+                    split_four(held[pass], part);
                     if (b + 1 < blocks) load(pass, b + 1);
                     const uint32_t at = w_at + (uint32_t)((b & 1) * STAGE_BYTES + pass * ROWS_A_PASS * 128);
 #pragma unroll
@@ -218,16 +283,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
             if (col < n) {
 #pragma unroll
                 for (int j = 0; j < SUM_COLS; ++j) {
-                    if (j < rows) *to = !partial && g > 0 ? __fadd_rn(*to, sum[j]) : sum[j];        // (this thread's own sum so far)
+                    if (j < rows) {
+                        const float total = !partial && g > 0 ? __fadd_rn(*to, sum[j]) : sum[j];    // (this thread's own sum so far)
+                        *to = total;
+                        if (!partial && !isfinite(total)) *not_finite = 1;          // (partial sums: when they are added up)
+                    }
                     to += ld;
                 }
             }
 #pragma unroll
             for (int j = 0; j < SUM_COLS; ++j) sum[j] = 0.0f;
         }
-        if (wild.x != 0.0f || wild.y != 0.0f)                              // (NaN: of one of the thread's rows)
-#pragma unroll
-            for (int pass = 0; pass < PASSES; ++pass) wild_rows[r0 + pass * ROWS_A_PASS] = 1;
     } else {
         // ---- copies of x, a block ahead, and products: of a block the smallest first
         const uint32_t idesc = instruction_descriptor_bf16(BW, nx, false);
@@ -276,33 +342,16 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
         while (clock64() - started < 400000) __nanosleep(1000);
     }
     pdl_wait();
-    if (threadIdx.x >= BW && threadIdx.x < 2 * BW) {
-        const int row = threadIdx.x - BW;
-        wild_rows[threadIdx.x] = row < nx && row0 + row < m && *reinterpret_cast<const volatile int*>(wild_x + row0 + row) != 0;
-    }
-    const int wild = threadIdx.x < 2 * BW && wild_rows[threadIdx.x] != 0;
-    if (__syncthreads_or(wild) && !gave_up) {
-        // of the rows of w that a thread has marked, those that hold such a value
-        for (int r = warp; r < BW; r += THREADS / 32) {
-            if (!wild_rows[r]) continue;
-            bool found = false;
-            for (int at = k_from + lane; at < k_to && col0 + r < n; at += 32)
-                found |= ((__float_as_uint(w[(int64_t)(col0 + r) * ldw + at]) + 0x8000u) & 0x7fffffffu) >= 0x7f800000u;
-            found = __any_sync(0xffffffffu, found);
-            if (lane == 0) wild_rows[r] = found;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < BW * nx; i += THREADS) {
-            const int local_col = i % BW, local_row = i / BW, col = col0 + local_col, row = row0 + local_row;
-            if (col >= n || row >= m || !(wild_rows[local_col] | wild_rows[BW + local_row])) continue;
-            float total = 0.0f;
-            for (int g = 0; k_from + g * GROUP < k_to; ++g) {
-                const float sum = plain_sum(a + (int64_t)row * lda, w + (int64_t)col * ldw, k_from + g * GROUP,
-                                            min(k_to, k_from + (g + 1) * GROUP));
-                if (partial) partial[((int64_t)(blockIdx.z * groups_per + g) * m + row) * n + col] = sum;
-                total = g == 0 ? sum : __fadd_rn(total, sum);
-            }
-            if (!partial) c[(int64_t)row * ldc + col] = total;
+    if (*not_finite && !gave_up && warp < WORK_WARPS) {
+        const int first = (warp >> 2) * SUM_COLS, col = col0 + (warp & 3) * 32 + lane;
+        const int rows_to = min(min(row0 + nx, row0 + first + SUM_COLS), m);
+        float* tile = reinterpret_cast<float*>(aligned) + warp * AGAIN_FLOATS<AGAIN_ROWS>;                // (the stages are free)
+        for (int row = row0 + first; row < rows_to; row += AGAIN_ROWS) {
+            unsigned again = 0;                                                         // of this thread's own elements
+            for (int i = 0; i < AGAIN_ROWS; ++i)
+                if (row + i < rows_to && col < n && !isfinite(c[(int64_t)(row + i) * ldc + col])) again |= 1u << i;
+            if (__any_sync(0xffffffffu, again))
+                sum_again<AGAIN_ROWS>(again, row, col, a, lda, w, ldw, c, ldc, m, k, nan_rows, tile);
         }
     }
     __syncthreads();
@@ -312,12 +361,36 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* wild_x,
     }
 }
 
+// What of c the warps of the kernel below have written and is not finite, summed again: a row of a warp's at a time.
+template <int VEC>
+__device__ __noinline__ void fold_again(float* c, int64_t ldc, int m, int n, const float* a, int64_t lda, const float* w,
+                                        int64_t ldw, int k, const int* nan_rows, float* tile) {
+    const int words = n / VEC, lane = threadIdx.x & 31;
+    const int64_t total = (int64_t)m * words;
+    for (int64_t from = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; from < total; from += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = min(from + lane, total - 1);
+        const int row = (int)(i / words), at = (int)(i % words) * VEC;
+        for (int j = 0; j < VEC; ++j) {
+            unsigned again = __ballot_sync(0xffffffffu, from + lane < total && !isfinite(c[(int64_t)row * ldc + at + j]));
+            while (again) {
+                const int of_row = __shfl_sync(0xffffffffu, row, __ffs(again) - 1);
+                const unsigned now = again & __ballot_sync(0xffffffffu, row == of_row);
+                again &= ~now;
+                sum_again<1>(now >> lane & 1, of_row, at + j, a, lda, w, ldw, c, ldc, m, k, nan_rows, tile);
+            }
+        }
+    }
+}
+
 // c = the sum of the groups' partial products, in ascending order; VEC neighbouring columns a thread.
 template <int VEC>
-__global__ void __launch_bounds__(256)
-fold_groups_kernel(const float* __restrict__ partial, int groups, float* __restrict__ c, int64_t ldc, int m, int n) {
+__global__ void __launch_bounds__(256, 4)
+fold_groups_kernel(const float* __restrict__ partial, int groups, float* c, int64_t ldc, int m, int n, const float* a, int64_t lda,
+                   const float* w, int64_t ldw, int k, const int* nan_rows) {
+    __shared__ __align__(16) float tiles[256 / 32][AGAIN_FLOATS<1>];
     const int words = n / VEC;
     const int64_t size = (int64_t)m * n, total = (int64_t)m * words;
+    bool again = false;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t row = total <= 0x7fffffff ? (uint32_t)i / (uint32_t)words : i / words;
         const int64_t at = (i - row * words) * VEC;
@@ -329,7 +402,10 @@ fold_groups_kernel(const float* __restrict__ partial, int groups, float* __restr
             for (int j = 0; j < VEC; ++j) sum[j] = __fadd_rn(sum[j], more[j]);
         }
         store_values<VEC>(c + row * ldc + at, sum);
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) again |= !isfinite(sum[j]);
     }
+    if (__any_sync(0xffffffffu, again)) fold_again<VEC>(c, ldc, m, n, a, lda, w, ldw, k, nan_rows, tiles[threadIdx.x / 32]);
 }
 
 struct Plan { int nx, tiles_x, groups, groups_per, splits; };
@@ -410,7 +486,7 @@ static int launch_range(const float* a, long long lda, const float* w, long long
     float* partial = plan.splits > 1 ? reinterpret_cast<float*>(scratch) : nullptr;
     uint8_t* parts = scratch + sum_bytes(plan, m, n);
     const long long kp = padded_k(k);
-    int* wild_x = reinterpret_cast<int*>(parts + 3 * m * kp * 2);
+    int* nan_rows = reinterpret_cast<int*>(parts + 3 * m * kp * 2);
     CUtensorMap map_x;
     {
         const cuuint64_t dims[3] = {(cuuint64_t)kp, (cuuint64_t)m, 3};
@@ -423,17 +499,17 @@ static int launch_range(const float* a, long long lda, const float* w, long long
     // The product's kernel reads w without waiting: the kernel that splits x, which it follows, starts behind all launches
     // before, unless none of those that may still run writes w.
     TvbLaunch split(dim3(m), dim3(128), 0, s, pdl && w_constant);
-    e = cudaLaunchKernelEx(&split.config, split_rows_kernel, a, (int64_t)lda, reinterpret_cast<uint2*>(parts), wild_x, m, k, (int)kp);
+    e = cudaLaunchKernelEx(&split.config, split_rows_kernel, a, (int64_t)lda, reinterpret_cast<uint2*>(parts), nan_rows, m, k, (int)kp);
     if (e != cudaSuccess) return (int)e;
     TvbLaunch launch(dim3((n + BW - 1) / BW, plan.tiles_x, plan.splits), dim3(THREADS), SHARED_BYTES, s, pdl);
-    e = cudaLaunchKernelEx(&launch.config, gemm_f32_tc_kernel, map_x, (const int*)wild_x, a, (int64_t)lda, w, (int64_t)ldw, c,
+    e = cudaLaunchKernelEx(&launch.config, gemm_f32_tc_kernel, map_x, (const int*)nan_rows, a, (int64_t)lda, w, (int64_t)ldw, c,
                            (int64_t)ldc, partial, plan.groups_per, m, n, k, plan.nx);
     if (e != cudaSuccess) return (int)e;
     if (plan.splits > 1) {
         const bool by_four = n % 4 == 0 && ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
         const int blocks = (int)std::min<long long>(((long long)m * n / (by_four ? 4 : 1) + 255) / 256, 8LL * sms);
-        if (by_four) fold_groups_kernel<4><<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n);
-        else fold_groups_kernel<1><<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n);
+        auto fold = by_four ? fold_groups_kernel<4> : fold_groups_kernel<1>;
+        fold<<<blocks, 256, 0, s>>>(partial, plan.groups, c, ldc, m, n, a, lda, w, ldw, k, nan_rows);
     }
     return tvb_last_error();
 }
