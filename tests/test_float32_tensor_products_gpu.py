@@ -112,13 +112,35 @@ def test_products_just_inside_float32(k):
     assert (got[inside].abs() <= bound(a, w)[inside]).all() and torch.equal(got[near], kernels.gemm_nt_simt(a, w)[near])
 
 
-@pytest.mark.parametrize("scale", [1e-30, 1e-18, 1e18, 1e30])
-def test_large_and_small_values(scale):
+@pytest.mark.parametrize("m,k", [(64, 512), (301, 2052)])
+@pytest.mark.parametrize("scale", [1e-42, 1e-40, 1e-38, 1e-36, 1e-34, 1e-30, 1e-18, 1e18, 1e26, 1e30, 1e36])
+@pytest.mark.parametrize("of_a", [True, False])
+def test_large_and_small_values(m, k, scale, of_a):
     generator = torch.Generator(device=DEV).manual_seed(3)
-    a, w = torch.randn(64, 512, generator=generator, device=DEV) * scale, torch.randn(96, 512, generator=generator, device=DEV)
+    a, w = torch.randn(m, k, generator=generator, device=DEV), torch.randn(96, k, generator=generator, device=DEV)
+    if of_a:
+        a *= scale
+    else:
+        w *= scale
     want = a.double() @ w.double().T
-    got = kernels.gemm_f32_tc(a, w).double()
-    assert ((got - want).abs() <= bound(a, w)).all()
+    got = kernels.gemm_f32_tc(a, w)
+    # below 2^-126 a sum of a group and theirs round to multiples of 2^-149
+    assert ((got.double() - want).abs() <= bound(a, w) + 2 * -(-k // 1024) * 2.0 ** -150).all()
+    if scale >= 1e36:                                       # sums beyond 2^96 are the float32 cores'
+        huge = want.abs() > 2.0 ** 97
+        assert huge.float().mean() > 0.9 and torch.equal(got[huge], kernels.gemm_nt_simt(a, w)[huge])
+
+
+@pytest.mark.parametrize("scales", [(1e-20, 1e-20), (1e-25, 1e-15), (1e-30, 1e-12), (1e-42, 1e3), (1e14, 1e14)])
+def test_products_at_the_ends_of_float32(scales):
+    """Both operands small, or both large: sums down to the smallest float32 and beyond 2^96."""
+    generator = torch.Generator(device=DEV).manual_seed(4)
+    a = torch.randn(64, 512, generator=generator, device=DEV) * scales[0]
+    w = torch.randn(96, 512, generator=generator, device=DEV) * scales[1]
+    want = a.double() @ w.double().T
+    for got in (kernels.gemm_f32_tc(a, w), kernels.gemm_f32_tc(a.repeat(3, 1), w)[128:]):
+        # (a product of two parts below 2^-149 / 2^32 is nothing to a multiple of 2^-149)
+        assert ((got.double() - want).abs() <= bound(a, w) + 2.0 ** -149).all()
 
 
 def test_which_kernel_takes_a_product():

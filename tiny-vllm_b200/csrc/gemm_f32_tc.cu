@@ -1,17 +1,18 @@
 // C[m, n] = A[m, k] . W[n, k]^T of float32 operands with more than a few rows, on the fifth-generation tensor cores
 // and with the precision of float32 sums.  (Few rows, and rows off the 16-byte boundary: gemm_simt.cu.)
 //
-// A float32 is the sum of three bfloat16, exactly: x1 is x rounded to 8 bits (so that the rest has either sign), x2 the
-// first 8 bits of the rest and x3 what is left.  A product of two such sums is nine products, of which the six largest
+// A float32 x times 2^16 is the sum of three bfloat16, exactly, from the smallest float32 to 2^111: x1 is rounded to 8 bits (so
+// that the rest has either sign), x2 the first 8 bits of the rest and x3 what is left.  (Without the factor the lowest bits of
+// operands below 2^-109 lie under bfloat16's smallest, 2^-133: an error of 5e-7 at 1e-34 and 3e-3 at 1e-38.)  The sums are
+// multiplied by 2^-32 when they leave the registers.  A product of two such sums is nine products, of which the six largest
 // are taken (x1 w1; x1 w2, x2 w1; x2 w2, x1 w3, x3 w1): what is left out is about 2^-26 of |x w|, with either sign.
 // Products of bfloat16 are exact in float32; the tensor cores add them up in tensor memory over 64 k, the small ones
 // first, and every such sum is then added by the float32 cores to a sum in registers, in ascending order of k: the
 // tensor cores cut off what does not fit instead of rounding it, which over all of k would shrink the sums.
 //
 // The sum of an output element has one order whatever m is: blocks of 64 k ascending inside a group of 1,024, the groups
-// ascending.  Infinities, NaN and values that round to infinity in bfloat16 have no such three parts, and the product of two
-// parts can be beyond float32 where x w is not (x1 and w1 round up) or is with one sign (x1 w2 has the other: NaN).  All of it
-// ends in a sum that is not finite: such an element is summed again by the float32 cores from the operands themselves, and has
+// ascending.  Infinities, NaN and values from 2^111 on have no such three parts, and a sum of 2^96 and more is beyond float32
+// with the factors (or NaN: x1 w2 may have the other sign than x1 w1).  All of it ends in a sum that is not finite: such an element is summed again by the float32 cores from the operands themselves, and has
 // their bits.
 //
 // x is split once, by a small kernel; w on its way into shared memory, by the 16 warps that also add up the sums: its
@@ -64,9 +65,17 @@ __device__ __forceinline__ float2 fma_two(float2 a, float2 b, float2 c) {
     return r.f;
 }
 
-// Four float32 as three times four bfloat16.
+constexpr float PART_SCALE = 65536.0f, SUM_SCALE = 1.0f / (PART_SCALE * PART_SCALE);
+
+__device__ __forceinline__ float2 scale_two(float2 a) {
+    union Pair { float2 f; unsigned long long u; } x{a}, y{make_float2(PART_SCALE, PART_SCALE)}, r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(x.u), "l"(y.u));
+    return r.f;
+}
+
+// Four float32 times 2^16 as three times four bfloat16.
 __device__ __forceinline__ void split_four(const float4& x, uint2* part) {
-    float2 rest[2] = {make_float2(x.x, x.y), make_float2(x.z, x.w)};
+    float2 rest[2] = {scale_two(make_float2(x.x, x.y)), scale_two(make_float2(x.z, x.w))};
     uint32_t* words = reinterpret_cast<uint32_t*>(part);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -102,10 +111,10 @@ static_assert(WORK_WARPS * AGAIN_FLOATS<AGAIN_ROWS> * 4 <= STAGES * STAGE_BYTES,
 
 // Elements of c that are not finite, of ROWS rows from `row` on and a column a lane (bit i of `again`: row + i), are summed again
 // from the operands by the float32 cores, in the order of gemm_simt.cu (segments of 128 k, a chain over the even and one over the
-// odd k of each; four segments a group, the groups ascending): those with infinities, and those where a part's product or a sum
-// of products is beyond float32 although theirs need not be.  A row of x with a NaN has nothing but NaN already.
+// odd k of each; four segments a group, the groups ascending): those with infinities, and those that are beyond float32 in parts
+// or with the parts' factors although theirs need not be.  A row of x with a NaN has nothing but NaN already.
 // What is left is finite again, or NaN from the next norm on, so that this runs rarely: 677 x 1,024 x 6,144 takes 61 us, with an
-// infinity in one row 87, all NaN 74, all infinities 920 (the float32 cores 261); 677 x 3,072 x 1,024, added up from partial
+// infinity in one row 87, all NaN 74, all infinities or beyond 2^96 920 (the float32 cores 261); 677 x 3,072 x 1,024, added up from partial
 // sums, 37, 460, 45 and 1,390 (139).
 template <int ROWS>
 __device__ __noinline__ void sum_again(unsigned again, int row, int col, const float* a, int64_t lda, const float* w, int64_t ldw,
@@ -284,7 +293,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_x, const int* nan_row
 #pragma unroll
                 for (int j = 0; j < SUM_COLS; ++j) {
                     if (j < rows) {
-                        const float total = !partial && g > 0 ? __fadd_rn(*to, sum[j]) : sum[j];    // (this thread's own sum so far)
+                        const float scaled = __fmul_rn(sum[j], SUM_SCALE);
+                        const float total = !partial && g > 0 ? __fadd_rn(*to, scaled) : scaled;    // (this thread's own sum so far)
                         *to = total;
                         if (!partial && !isfinite(total)) *not_finite = 1;          // (partial sums: when they are added up)
                     }
