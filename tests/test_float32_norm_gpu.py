@@ -4,7 +4,7 @@ the launch before writes (of the norm and of products of a few rows)."""
 import pytest
 import torch
 
-from tinyvllm_b200.ops import kernels
+from tinyvllm_b200.ops import kernels, linear, linear_into_stream, linear_silu
 
 pytestmark = pytest.mark.gpu
 
@@ -43,6 +43,29 @@ def test_weights_and_products_of_the_launch_before_are_awaited(width):
         kernels.rms_norm(x, weight, 1e-6, out=made)
         got = kernels.gemm_nt_simt(rows, made[2900:])                # a weight that the launch before writes
         assert torch.equal(got, kernels.gemm_nt_simt(rows, made[2900:].clone())), turn
+
+
+@pytest.mark.parametrize("rows", [1, 5, 8, 20, 64, 200])
+def test_linear_awaits_a_weight_that_the_launch_before_writes(rows):
+    """Without weight_constant a weight may come from the launch before, whatever kernel takes the product."""
+    generator = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(6000, 1024, generator=generator, device="cuda")
+    few = torch.randn(rows, 1024, generator=generator, device="cuda")
+    made = torch.empty_like(x)
+    for turn in range(30):
+        made.fill_(50.0)
+        norm = torch.randn(1024, generator=generator, device="cuda")
+        kernels.rms_norm(x, norm, 1e-6, out=made)              # (lets what is launched behind it begin early)
+        got = linear(few, made[5000:])
+        assert torch.equal(got, linear(few, made[5000:].clone())), turn
+    made.fill_(50.0)
+    kernels.rms_norm(x, norm, 1e-6, out=made)
+    got = linear_silu(few, made[5000:])
+    assert torch.equal(got, linear_silu(few, made[5000:].clone()))
+    made.fill_(50.0)
+    kernels.rms_norm(x, norm, 1e-6, out=made)
+    got = linear_into_stream(few, made[4976:], few)[0]
+    assert torch.equal(got, linear_into_stream(few, made[4976:].clone(), few)[0])
 
 
 @pytest.mark.parametrize("inter", [1, 6, 8, 1020, 1028, 3072])

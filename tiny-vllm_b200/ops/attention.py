@@ -455,7 +455,7 @@ def latent_attention(ctx, mixer, projected: torch.Tensor, run: int) -> torch.Ten
         pairing=pairing)
     from .linear import linear
 
-    q = linear(q_latent, mixer.uq_weight).view(tokens, heads, mixer.key_dim + rot)
+    q = linear(q_latent, mixer.uq_weight, weight_constant=True).view(tokens, heads, mixer.key_dim + rot)
     folded = torch.empty((tokens, heads, rank + rot), dtype=projected.dtype, device=projected.device)
     kernels.head_product(q[:, :, :mixer.key_dim], mixer.uk_by_head, folded[:, :, :rank])
     if rot > 0:

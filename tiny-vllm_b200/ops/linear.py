@@ -17,16 +17,18 @@ from . import kernels
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, *, out_dtype: torch.dtype | None = None,
-           out: torch.Tensor | None = None) -> torch.Tensor:
+           out: torch.Tensor | None = None, weight_constant: bool = False) -> torch.Tensor:
     """x [m, k] times weight [n, k] transposed; the result has ``out_dtype``
-    (default: the dtype of x).  ``weight`` is a parameter, which the kernels may read before the one before them ends."""
+    (default: the dtype of x).  ``weight_constant``: nothing in flight on the stream writes the weight (a model's, loaded
+    long ago), so that float32 products may read it while the kernel before them still runs.  (bfloat16 products of few
+    rows always do.)"""
     if not x.is_cuda:
         raise kernels.KernelError("linear runs on CUDA tensors only; there is no CPU path")
     out_dtype = out_dtype or x.dtype
     if x.dtype == torch.float32:
         if out_dtype != torch.float32:
             raise kernels.KernelError("a float32 product has a float32 result")
-        return _linear_f32(x, weight, out)
+        return _linear_f32(x, weight, out, weight_constant)
     from . import gemm
 
     return gemm.linear_bf16(x, weight, out_dtype=out_dtype, out=out)
@@ -38,18 +40,19 @@ def linear(x: torch.Tensor, weight: torch.Tensor, *, out_dtype: torch.dtype | No
 F32_CORE_ROWS = 32
 
 
-def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None) -> torch.Tensor:
+def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None, weight_constant: bool) -> torch.Tensor:
     if x.shape[0] > F32_CORE_ROWS and kernels.gemm_f32_tc_takes(x, weight):
-        return kernels.gemm_f32_tc(x, weight, out=out, weight_constant=True)
-    return kernels.gemm_nt_simt(x, weight, out=out, weight_constant=True)
+        return kernels.gemm_f32_tc(x, weight, out=out, weight_constant=weight_constant)
+    return kernels.gemm_nt_simt(x, weight, out=out, weight_constant=weight_constant)
 
 
-def linear_silu(x: torch.Tensor, gate_up_weight: torch.Tensor) -> torch.Tensor:
-    """round(round(silu(x . gate^T)) * (x . up^T)) for a packed [gate | up] weight, [m, inter]."""
+def linear_silu(x: torch.Tensor, gate_up_weight: torch.Tensor, *, weight_constant: bool = False) -> torch.Tensor:
+    """round(round(silu(x . gate^T)) * (x . up^T)) for a packed [gate | up] weight, [m, inter].  ``weight_constant``: as in
+    :func:`linear`."""
     if not x.is_cuda:
         raise kernels.KernelError("linear_silu runs on CUDA tensors only; there is no CPU path")
     if x.dtype == torch.float32:
-        return kernels.silu_mul(_linear_f32(x, gate_up_weight, None))
+        return kernels.silu_mul(_linear_f32(x, gate_up_weight, None, weight_constant))
     from . import gemm
 
     return gemm.linear_silu_bf16(x, gate_up_weight)
@@ -65,8 +68,9 @@ FUSED_NORM_MAX_ROWS = int(os.environ.get("TINYVLLM_B200_FUSED_NORM_ROWS", "2"))
 STREAM_ADD = os.environ.get("TINYVLLM_B200_STREAM_ADD", "1") != "0"
 
 
-def linear_into_stream(x: torch.Tensor, weight: torch.Tensor, stream: torch.Tensor):
-    """A part's output projection, added to the residual stream where that saves a kernel.
+def linear_into_stream(x: torch.Tensor, weight: torch.Tensor, stream: torch.Tensor, *, weight_constant: bool = False):
+    """A part's output projection, added to the residual stream where that saves a kernel.  ``weight_constant``: as in
+    :func:`linear`.
 
     Returns (None, stream + linear(x, weight)) when the product's kernel does the addition on its
     way out (small bfloat16 batches): the new stream then carries ``row_squares``, the sums of
@@ -84,17 +88,18 @@ def linear_into_stream(x: torch.Tensor, weight: torch.Tensor, stream: torch.Tens
                                                prefetch=gemm.next_weight(weight))
         summed.row_squares = squares
         return None, summed
-    return linear(x, weight), stream
+    return linear(x, weight, weight_constant=weight_constant), stream
 
 
 def linear_norm(hidden: torch.Tensor | None, residual: torch.Tensor | None, norm, weight: torch.Tensor, *,
-                silu: bool = False):
+                silu: bool = False, weight_constant: bool = False):
     """(linear(norm(hidden + residual), weight), hidden + residual): a pre-norm and the
     projection behind it as one operation.  ``norm`` is a norm part (``weight``, ``eps``,
     ``forward``, ``add``).  Without a residual the stream is ``hidden`` itself; without
     ``hidden`` (None) the residual holds the sum already (:func:`linear_into_stream`).  ``silu``
     applies SiLU(gate) * up to a packed [gate | up] weight.  Small bfloat16 batches run as
-    one kernel; everything else as the norm kernel and the product."""
+    one kernel; everything else as the norm kernel and the product.  ``weight_constant``: as in
+    :func:`linear`."""
     from . import gemm
 
     if hidden is None:
@@ -107,7 +112,7 @@ def linear_norm(hidden: torch.Tensor | None, residual: torch.Tensor | None, norm
                                        row_squares=squares, prefetch=gemm.next_weight(weight))
             return out, residual
         x = norm.forward(residual)
-        return (linear_silu(x, weight) if silu else linear(x, weight)), residual
+        return (linear_silu if silu else linear)(x, weight, weight_constant=weight_constant), residual
     if (hidden.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and hidden.is_contiguous()
             and getattr(norm, "folds_into_product", False) and gemm.small(hidden, weight)
             and hidden.shape[0] <= FUSED_NORM_MAX_ROWS
@@ -121,4 +126,4 @@ def linear_norm(hidden: torch.Tensor | None, residual: torch.Tensor | None, norm
         x, stream = norm.forward(hidden), hidden
     else:
         x, stream = norm.add(hidden, residual)
-    return (linear_silu(x, weight) if silu else linear(x, weight)), stream
+    return (linear_silu if silu else linear)(x, weight, weight_constant=weight_constant), stream

@@ -80,16 +80,16 @@ class GQAAttention(Part):
 
     # ---------------------------------------------------------------- running
     def forward(self, x, ctx, run: int):
-        qkv = linear(x, self.qkv_weight)
+        qkv = linear(x, self.qkv_weight, weight_constant=True)
         attended = attention_ops.mixer_attention(ctx, self, qkv, run)
-        return linear(attended, self.o_weight)
+        return linear(attended, self.o_weight, weight_constant=True)
 
     def forward_normed(self, hidden, residual, norm, ctx, run: int):
         """forward(norm(hidden + residual)) and the new residual stream; the output is None when
         the output projection has added it to the stream itself."""
-        qkv, residual = linear_norm(hidden, residual, norm, self.qkv_weight)
+        qkv, residual = linear_norm(hidden, residual, norm, self.qkv_weight, weight_constant=True)
         attended = attention_ops.mixer_attention(ctx, self, qkv, run)
-        return linear_into_stream(attended, self.o_weight, residual)
+        return linear_into_stream(attended, self.o_weight, residual, weight_constant=True)
 
 
 def distance_buckets(rows: int, far: float) -> list[int]:
@@ -362,10 +362,10 @@ class WindowedAttention(Part):
         attention_ops.windowed_attention(ctx, self, projected, at, run, out)
 
     def forward(self, x, ctx, run: int):
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         attended = torch.empty((x.shape[0], self.out_cols), dtype=x.dtype, device=x.device)
         self.between(projected, 0, ctx, attended, run)
-        y = linear(attended, self.o_weight, out_dtype=self.out_dtype)
+        y = linear(attended, self.o_weight, out_dtype=self.out_dtype, weight_constant=True)
         return y if self.output_bias is None else kernels.add_row_bias(y, self.output_bias)
 
 
@@ -478,9 +478,9 @@ class LatentAttention(Part):
                    kernels.attention_tiles_singles_floats(rows, self.num_heads, self.kv_rank, self.window, 0, span))
 
     def forward(self, x, ctx, run: int):
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         gated = attention_ops.latent_attention(ctx, self, projected, run)
-        return linear(gated, self.o_weight, out_dtype=self.out_dtype)
+        return linear(gated, self.o_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 register_part("mixer", "gqa_attention", GQAAttention)

@@ -116,7 +116,7 @@ class ParallelResidualBlock(Block):
             if self.feed_forward is not None:
                 update = kernels.sum_pair(update, self.feed_forward.forward(x, ctx))
             return update, residual
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         inner = torch.empty((x.shape[0], self.out_weight.shape[1]), dtype=x.dtype, device=x.device)
         at_in = at_out = 0
         for part in self.guests:
@@ -128,7 +128,7 @@ class ParallelResidualBlock(Block):
                 part.between(projected, at_in, ctx, out)
             at_in += sum(rows for _, rows in part.input_rows())
             at_out += columns
-        return linear(inner, self.out_weight, out_dtype=torch.float32), residual
+        return linear(inner, self.out_weight, out_dtype=torch.float32, weight_constant=True), residual
 
 
 class PostNormResidualBlock(Block):

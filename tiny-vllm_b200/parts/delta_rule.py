@@ -112,7 +112,7 @@ class GatedDeltaRule(Part):
 
     # ---------------------------------------------------------------- running
     def forward(self, x, ctx, run: int):
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         entries = dict(row_starts=ctx.row_starts, state_slots=ctx.state_slots, token_row=ctx.token_row)
         mixed = kernels.short_convolution(projected[:, :self.conv_cols], self.conv_by_tap, bias=None, act="silu",
                                           state=ctx.storage.state_of(run, self.conv_state), **entries)
@@ -124,7 +124,7 @@ class GatedDeltaRule(Part):
             unit_eps=self.unit_eps, unit_norm=self.out_norm is not None, norm_weight=self.norm_weight, eps=self.eps,
             gate_at=None if self.gate is None else self.conv_cols, gate_act=self.gate,
             state=ctx.storage.state_of(run, self.delta_state), **entries)
-        return linear(gated, self.o_weight, out_dtype=self.out_dtype)
+        return linear(gated, self.o_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 register_part("mixer", "gated_delta_rule", GatedDeltaRule)

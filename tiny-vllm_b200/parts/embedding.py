@@ -92,7 +92,7 @@ class LMHead(Part):
         return [self.weight]
 
     def forward(self, hidden_rows):
-        logits = linear(hidden_rows, self.weight, out_dtype=torch.float32)
+        logits = linear(hidden_rows, self.weight, out_dtype=torch.float32, weight_constant=True)
         return logits if self.scale == 1.0 else kernels.scale_float32(logits, self.scale)
 
 

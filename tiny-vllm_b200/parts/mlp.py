@@ -68,12 +68,12 @@ class SwiGLU(Part):
     # ------------------------------------------------------------ on its own
     def _activated(self, x):
         if self.activation == "silu":
-            return linear_silu(x, self.gate_up_weight)
-        return kernels.gated_act(linear(x, self.gate_up_weight), 0, self.intermediate_size,
+            return linear_silu(x, self.gate_up_weight, weight_constant=True)
+        return kernels.gated_act(linear(x, self.gate_up_weight, weight_constant=True), 0, self.intermediate_size,
                                  self.intermediate_size, self.activation)
 
     def forward(self, x, ctx):
-        return linear(self._activated(x), self.down_weight, out_dtype=self.out_dtype)
+        return linear(self._activated(x), self.down_weight, out_dtype=self.out_dtype, weight_constant=True)
 
     def forward_normed(self, hidden, residual, norm, ctx):
         """forward(norm(hidden + residual)) and the new residual stream; the output is None when
@@ -86,8 +86,8 @@ class SwiGLU(Part):
             else:
                 x, residual = norm.add(hidden, residual)
             return self.forward(x, ctx), residual
-        activated, residual = linear_norm(hidden, residual, norm, self.gate_up_weight, silu=True)
-        return linear_into_stream(activated, self.down_weight, residual)
+        activated, residual = linear_norm(hidden, residual, norm, self.gate_up_weight, silu=True, weight_constant=True)
+        return linear_into_stream(activated, self.down_weight, residual, weight_constant=True)
 
 
 register_part("feed_forward", "swiglu", SwiGLU)
@@ -138,10 +138,10 @@ class RoutedExperts(Part):
         return [self.up_weight, self.down_weight]
 
     def forward(self, x, ctx):
-        logits = linear(x, self.router_weight, out_dtype=torch.float32)
-        inner = kernels.route_act(logits, linear(x, self.up_weight), experts=self.experts, top=self.top,
+        logits = linear(x, self.router_weight, out_dtype=torch.float32, weight_constant=True)
+        inner = kernels.route_act(logits, linear(x, self.up_weight, weight_constant=True), experts=self.experts, top=self.top,
                                   ff=self.ff, shared_ff=self.shared_ff, activation=self.activation)
-        return linear(inner, self.down_weight, out_dtype=self.out_dtype)
+        return linear(inner, self.down_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 register_part("feed_forward", "routed_experts", RoutedExperts)
@@ -209,13 +209,13 @@ class GatedRoutedExperts(Part):
         return [self.in_weight, self.down_weight]
 
     def forward(self, x, ctx):
-        logits = linear(x, self.router_weight, out_dtype=torch.float32)
+        logits = linear(x, self.router_weight, out_dtype=torch.float32, weight_constant=True)
         inner = kernels.route_gated_act(
-            logits, linear(x, self.in_weight), experts=self.experts, top=self.top, ff=self.ff,
+            logits, linear(x, self.in_weight, weight_constant=True), experts=self.experts, top=self.top, ff=self.ff,
             shared_ff=self.shared_ff, limit=self.limit, shared_limit=self.shared_limit, alpha=self.alpha,
             route_scale=self.route_scale, correction=self.correction, groups=self.groups, keep=self.keep,
             shared_gated=self.shared_gate)
-        return linear(inner, self.down_weight, out_dtype=self.out_dtype)
+        return linear(inner, self.down_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 register_part("feed_forward", "gated_routed_experts", GatedRoutedExperts)
@@ -288,12 +288,12 @@ class SoftmaxRoutedExperts(Part):
     def forward_carried(self, x, ctx):
         """(y, row_scale): the part's output is y + row_scale[:, None] * x; ``row_scale`` (float32 [tokens], the
         weights of the chosen pass-through slots) is None where the part has no such slots."""
-        logits = linear(x, self.router_weight, out_dtype=torch.float32)
+        logits = linear(x, self.router_weight, out_dtype=torch.float32, weight_constant=True)
         inner, passed = kernels.route_softmax_gated(
-            logits, linear(x, self.in_weight), experts=self.experts, identity=self.identity, top=self.top,
+            logits, linear(x, self.in_weight, weight_constant=True), experts=self.experts, identity=self.identity, top=self.top,
             ff=self.ff, correction=self.correction, renormalise=self.renormalise, groups=self.groups, keep=self.keep,
             limit=self.limit, alpha=self.alpha)
-        return linear(inner, self.down_weight, out_dtype=self.out_dtype), passed
+        return linear(inner, self.down_weight, out_dtype=self.out_dtype, weight_constant=True), passed
 
     def forward(self, x, ctx):
         y, passed = self.forward_carried(x, ctx)

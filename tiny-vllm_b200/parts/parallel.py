@@ -66,12 +66,12 @@ class ParallelMixers(Part):
 
     # ---------------------------------------------------------------- running
     def forward_pair(self, x, ctx, run: int) -> NormedPair:
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         outputs, at = [], 0
         for guest, o_weight in ((self.left, self.left_o_weight), (self.right, self.right_o_weight)):
             inner = torch.empty((x.shape[0], o_weight.shape[1]), dtype=x.dtype, device=x.device)
             guest.between(projected, at, ctx, inner, run)
-            outputs.append(linear(inner, o_weight, out_dtype=torch.float32))
+            outputs.append(linear(inner, o_weight, out_dtype=torch.float32, weight_constant=True))
             at += sum(rows for _, rows in guest.input_rows())
         return NormedPair(outputs[0], outputs[1], left_weight=self.left_norm_weight,
                           right_weight=self.right_norm_weight, left_bias=getattr(self.left, "output_bias", None),

@@ -83,7 +83,7 @@ class LinearRecurrentUnit(Part):
     # ---------------------------------------------------------------- running
     def forward(self, x, ctx, run: int):
         c = self.channels
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         entries = dict(row_starts=ctx.row_starts, state_slots=ctx.state_slots, token_row=ctx.token_row)
         u = kernels.short_convolution(projected[:, :c], self.conv_by_tap, bias=self.conv_bias, act=None,
                                       in_bias=self.x_bias, state=ctx.storage.state_of(run, self.conv_state), **entries)
@@ -94,7 +94,7 @@ class LinearRecurrentUnit(Part):
             bias_y=self.y_bias, act=self.activation, state=ctx.storage.state_of(run, self.unit_state), single=single,
             pre=None if fused else kernels.block_products(u, self.gate_weight),
             weight=self.gate_weight if fused else None, **entries)
-        return linear(mixed, self.o_weight, out_dtype=self.out_dtype)
+        return linear(mixed, self.o_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 register_part("mixer", "linear_recurrent_unit", LinearRecurrentUnit)

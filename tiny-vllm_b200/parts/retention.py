@@ -82,7 +82,7 @@ class Retention(Part):
 
     # ---------------------------------------------------------------- running
     def forward(self, x, ctx, run: int):
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         position = self.position
         v_at = 2 * self.qk_cols
         gated = kernels.retention(
@@ -94,7 +94,7 @@ class Retention(Part):
             rot_dims=0 if position is None else position.rot_dims,
             pairing="half_split" if position is None else position.pairing, key_scale=self.key_scale,
             unit_norm=self.unit_norm, eps=self.eps, gate_act=self.gate)
-        return linear(gated, self.o_weight, out_dtype=self.out_dtype)
+        return linear(gated, self.o_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 class GatedRecurrence(Part):
@@ -171,14 +171,14 @@ class GatedRecurrence(Part):
         return True                  # no attention over pages: any cutting of a step into tiles will do
 
     def forward(self, x, ctx, run: int):
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         normed = kernels.gated_recurrence(
             projected, q_at=0, g_at=self.qk_cols, v_at=2 * self.qk_cols, heads=self.num_heads, dim=self.key_dim,
             vdim=self.value_dim, state=ctx.storage.state_of(run), row_starts=ctx.row_starts,
             state_slots=ctx.state_slots, token_row=ctx.token_row, bias=self.gate_bias, lower=self.lower,
             query_act=self.query_act, unit_norm=self.out_norm is not None, norm_weight=self.norm_weight,
             eps=self.eps)
-        return linear(normed, self.o_weight, out_dtype=self.out_dtype)
+        return linear(normed, self.o_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 class GatedLinearAttention(Part):
@@ -268,13 +268,13 @@ class GatedLinearAttention(Part):
         return True                  # no attention over pages: any cutting of a step into tiles will do
 
     def forward(self, x, ctx, run: int):
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         v_at = 2 * self.qk_cols
         decays = {}
         if ctx.num_tokens == ctx.num_rows and kernels.gated_step_takes(self.value_dim):
             decays = dict(low_at=self.low_at, low_weight=self.a2_weight)     # the step kernel does the second step itself
         else:
-            decays = dict(gate_pre=linear(projected[:, self.low_at:], self.a2_weight, out_dtype=torch.float32))
+            decays = dict(gate_pre=linear(projected[:, self.low_at:], self.a2_weight, out_dtype=torch.float32, weight_constant=True))
         gated = kernels.gated_recurrence(
             projected, q_at=0, g_at=-1, k_at=self.qk_cols, v_at=v_at, heads=self.num_heads, dim=self.key_dim,
             vdim=self.value_dim, state=ctx.storage.state_of(run), row_starts=ctx.row_starts,
@@ -282,7 +282,7 @@ class GatedLinearAttention(Part):
             query_scale=self.query_scale, gate_exponent=self.decay_exponent, unit_norm=self.out_norm is not None,
             norm_weight=self.norm_weight, eps=self.eps,
             out_gate_at=None if self.gate is None else v_at + self.out_cols, out_gate_act=self.gate, **decays)
-        return linear(gated, self.o_weight, out_dtype=self.out_dtype)
+        return linear(gated, self.o_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 register_part("mixer", "retention", Retention)

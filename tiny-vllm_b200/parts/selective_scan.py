@@ -102,11 +102,11 @@ class SelectiveScan(Part):
         entries = dict(row_starts=ctx.row_starts, state_slots=ctx.state_slots, token_row=ctx.token_row)
         x = kernels.short_convolution(projected[:, at:at + inner], self.conv_by_tap, bias=self.conv_bias, act="silu",
                                       state=ctx.storage.state_of(run, self.conv_state), **entries)
-        mixed = linear(x, self.x_weight)
+        mixed = linear(x, self.x_weight, weight_constant=True)
         low = mixed[:, :rank]
         single = ctx.num_tokens == ctx.num_rows               # a step of single tokens
         fused = single and kernels.selective_step_takes(ctx.num_rows, rank)
-        pre = None if fused else linear(low, self.dt_weight, out_dtype=torch.float32)
+        pre = None if fused else linear(low, self.dt_weight, out_dtype=torch.float32, weight_constant=True)
         kernels.selective_scan(
             x, pre=pre, low=low if fused else None, dt_weight=self.dt_weight if fused else None,
             z=projected[:, at + inner:at + 2 * inner], b=mixed[:, rank:rank + self.state],
@@ -114,10 +114,10 @@ class SelectiveScan(Part):
             state=ctx.storage.state_of(run, self.scan_state), out=out, single=single, **entries)
 
     def forward(self, x, ctx, run: int):
-        projected = linear(x, self.in_weight)
+        projected = linear(x, self.in_weight, weight_constant=True)
         inner = torch.empty((x.shape[0], self.inner), dtype=x.dtype, device=x.device)
         self.between(projected, 0, ctx, inner, run)
-        return linear(inner, self.o_weight, out_dtype=self.out_dtype)
+        return linear(inner, self.o_weight, out_dtype=self.out_dtype, weight_constant=True)
 
 
 register_part("mixer", "selective_scan", SelectiveScan)
