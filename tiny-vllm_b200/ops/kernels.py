@@ -1895,6 +1895,16 @@ def gemm_f32_scratch_floats(m: int, n: int, k: int) -> int:
     return _fn("gemm_simt", "tvb_gemm_f32_scratch_floats", [c_int, c_int, c_int], c_longlong)(m, n, k)
 
 
+def gemm_f32_us(m: int, n: int, k: int) -> float:
+    """About what :func:`gemm_nt_simt` takes for a float32 product of more than 8 rows, in microseconds."""
+    return _fn("gemm_simt", "tvb_gemm_f32_us", [c_int, c_int, c_int], ctypes.c_double)(m, n, k)
+
+
+def gemm_f32_tc_us(m: int, n: int, k: int) -> float:
+    """About what :func:`gemm_f32_tc` takes, in microseconds."""
+    return _fn("gemm_f32_tc", "tvb_gemm_f32_tc_us", [c_int, c_int, c_int], ctypes.c_double)(m, n, k)
+
+
 def gemm_f32_tc_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether :func:`gemm_f32_tc` takes this product: float32, rows contiguous and on 16-byte boundaries, k a
     multiple of 4."""

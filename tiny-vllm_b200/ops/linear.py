@@ -1,7 +1,8 @@
 """x . W^T for the parts, by storage dtype.
 
-float32: the package's own kernels, true 32-bit: up to F32_CORE_ROWS rows on the float32 cores, more on the tensor
-cores with every operand as three bfloat16 (each of the two gives a row the same bits whatever else is in the batch).
+float32: the package's own kernels, true 32-bit: up to F32_CORE_ROWS rows and narrow products on the float32 cores, the others
+on the tensor cores with every operand as three bfloat16 (each of the two gives a row the same bits whatever else is in the
+batch).
 bfloat16: the tensor-core kernels of this package where they take the shape,
 else cuBLAS through ``torch.nn.functional.linear``, which is what the
 reference's engine calls for every projection (tinyvllm/layers.py:84-85).
@@ -9,6 +10,7 @@ reference's engine calls for every projection (tinyvllm/layers.py:84-85).
 
 from __future__ import annotations
 
+import functools
 import os
 
 import torch
@@ -38,10 +40,24 @@ def linear(x: torch.Tensor, weight: torch.Tensor, *, out_dtype: torch.dtype | No
 # products at any number of rows up to 128 (a CTA walks 1,024 k in 16 steps of 1.2 us), the float32 cores 16 to 24 us
 # for 32 rows, 29 to 42 us for 48.
 F32_CORE_ROWS = 32
+# Smallest k of the tensor cores.  Their error against 64 bits is larger below (operands of either sign, k = 4 / 8 / 16: 4.9e-8,
+# 4.9e-8, 5.0e-8; float32 cores 4.1e-8, 4.8e-8, 6.0e-8).
+F32_TENSOR_K = 16
+
+
+@functools.lru_cache(maxsize=4096)
+def _tensor_cores_are_quicker(rows: int, columns: int, k: int) -> bool:
+    """Whether the tensor cores take a float32 product of more than F32_CORE_ROWS rows, by the two kernels' estimates.  The
+    float32 cores are quicker where one round of their tiles holds all of a narrow or short product: splitting x, a launch
+    more, and columns up to 128 are then not paid back.  Measured (us, float32 cores / tensor cores): 301 x 512 x 64 5.3 /
+    6.3, 8,192 x 128 x 64 7.6 / 15.2, 2,048 x 64 x 2,048 29 / 34, 8,192 x 64 x 4,096 127 / 176; but 301 x 64 x 512 27 /
+    15, 677 x 128 x 1,024 28.7 / 27.0, 2,048 x 256 x 2,048 76 / 35."""
+    return k >= F32_TENSOR_K and kernels.gemm_f32_tc_us(rows, columns, k) < kernels.gemm_f32_us(rows, columns, k)
 
 
 def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None, weight_constant: bool) -> torch.Tensor:
-    if x.shape[0] > F32_CORE_ROWS and kernels.gemm_f32_tc_takes(x, weight):
+    if (x.shape[0] > F32_CORE_ROWS and kernels.gemm_f32_tc_takes(x, weight)
+            and _tensor_cores_are_quicker(x.shape[0], weight.shape[0], x.shape[1])):
         return kernels.gemm_f32_tc(x, weight, out=out, weight_constant=weight_constant)
     return kernels.gemm_nt_simt(x, weight, out=out, weight_constant=weight_constant)
 
