@@ -13,7 +13,8 @@ DEV = "cuda:0"
 
 def bound(a, w):
     """A block of 64 k: 4 products that the tensor cores cut at 2^-23 of the sum so far (twice, for the small ones before
-    them), then one rounding a block and a group; the parts left out are 2^-24 of a product at most."""
+    them), then one rounding a block and a group; the parts left out, x2 w3 and x3 w2, are 2^-8 2^-16 of a product each at
+    most, together 2 units of 2^-24."""
     k = a.shape[1]
     return (8 * 2.0 ** -23 + (-(-min(k, 1024) // 64) + -(-k // 1024) + 2) * 2.0 ** -24) * (a.double().abs() @ w.double().abs().T)
 
@@ -34,6 +35,66 @@ def test_sums_are_within_float32_and_the_same_in_every_batch(n, k):
     kernels.gemm_f32_tc(apart, w, out=into[:, 2:n + 2])
     assert torch.equal(into[:, 2:n + 2], whole) and (into[:, :2] == 7.0).all() and (into[:, n + 2:] == 7.0).all()
     assert kernels.gemm_f32_tc_status() == 0
+
+
+def draw_operands(kind, n, k, generator):
+    def normal(rows):
+        return torch.randn(rows, k, generator=generator, device=DEV)
+
+    def uniform(rows):
+        return torch.rand(rows, k, generator=generator, device=DEV)
+
+    if kind == "normal":
+        return normal(n), normal(n) * 0.02
+    if kind == "long tails":
+        return normal(n) * torch.exp(2 * normal(n)), normal(n) * 0.02
+    if kind == "one sign by either":
+        return uniform(n), normal(n)
+    if kind == "one sign":
+        return uniform(n), uniform(n)
+    if kind == "one sign, long tails":
+        return torch.exp(2 * normal(n)), torch.exp(2 * normal(n))
+    if kind == "rows of one value":
+        return (uniform(n)[:, :1] + 0.5).expand(n, k).contiguous(), (uniform(n)[:, :1] + 0.5).expand(n, k).contiguous()
+    # every part left out has the sign and nearly the size of the largest there is
+    return (torch.full((n, k), 1.0 + 2.0 ** -8 - 2.0 ** -23, device=DEV),) * 2
+
+
+@pytest.mark.parametrize("k", [4, 12, 16, 64, 128, 1024, 2052])
+@pytest.mark.parametrize("kind", ["normal", "long tails", "one sign by either", "one sign", "one sign, long tails", "rows of one value",
+                                  "largest left out"])
+def test_error_against_64_bits_beside_the_float32_cores(kind, k):
+    generator = torch.Generator(device=DEV).manual_seed(k)
+    a, w = draw_operands(kind, 256, k, generator)
+    want = a.double() @ w.double().T
+    errors = []
+    for product in (kernels.gemm_f32_tc, kernels.gemm_nt_simt):
+        off = product(a, w).double() - want
+        assert product is kernels.gemm_nt_simt or (off.abs() <= bound(a, w)).all()
+        errors.append((off.norm() / want.norm()).item())
+    # weights of either sign, as a model's: no further off than the float32 cores from the k on that the tensor cores take
+    # (measured 0.44 to 0.98 of it; long tails at 64 k hang on few products: 1.07)
+    if kind in ("normal", "one sign by either") and k >= 16 or kind in ("long tails", "rows of one value") and k >= 128:
+        assert errors[0] <= errors[1], errors
+
+
+def test_sums_that_fit_24_bits_are_exact():
+    generator = torch.Generator(device=DEV).manual_seed(8)
+    a, w = (torch.randint(-50, 51, (130, 3072), generator=generator, device=DEV).float() for _ in range(2))
+    assert torch.equal(kernels.gemm_f32_tc(a, w).double(), a.double() @ w.double().T)
+    x = torch.randn(70, 256, generator=generator, device=DEV) * 1e-20
+    assert torch.equal(kernels.gemm_f32_tc(x, torch.eye(256, device=DEV)), x)
+
+
+def test_rounding_changes_where_the_kernel_does():
+    """32 rows are the float32 cores', 33 the tensor cores': a row differs by no more than both kernels' errors."""
+    generator = torch.Generator(device=DEV).manual_seed(9)
+    a, w = torch.randn(33, 1024, generator=generator, device=DEV), torch.randn(1024, 1024, generator=generator, device=DEV)
+    few, more = linear(a[:32], w), linear(a, w)[:32]
+    assert torch.equal(few, kernels.gemm_nt_simt(a[:32], w)) and torch.equal(more, kernels.gemm_f32_tc(a, w)[:32])
+    # a chain of 64 products, the sum of two chains, 3 segments and 2 groups on the float32 cores
+    cores = (64 + 1 + 3 + 2) * 2.0 ** -24 * (a[:32].double().abs() @ w.double().abs().T)
+    assert ((few.double() - more.double()).abs() <= cores + bound(a[:32], w)).all()
 
 
 @pytest.mark.parametrize("k", [64, 2048])

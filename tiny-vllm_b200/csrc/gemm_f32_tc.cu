@@ -1,19 +1,27 @@
 // C[m, n] = A[m, k] . W[n, k]^T of float32 operands with more than a few rows, on the fifth-generation tensor cores
-// and with the precision of float32 sums.  (Few rows, and rows off the 16-byte boundary: gemm_simt.cu.)
+// and with all 24 bits of the operands.  (Few rows, narrow products, and rows off the 16-byte boundary: gemm_simt.cu.)
 //
 // A float32 x times 2^16 is the sum of three bfloat16, exactly, from the smallest float32 to 2^111: x1 is rounded to 8 bits (so
 // that the rest has either sign), x2 the first 8 bits of the rest and x3 what is left.  (Without the factor the lowest bits of
 // operands below 2^-109 lie under bfloat16's smallest, 2^-133: an error of 5e-7 at 1e-34 and 3e-3 at 1e-38.)  The sums are
 // multiplied by 2^-32 when they leave the registers.  A product of two such sums is nine products, of which the six largest
-// are taken (x1 w1; x1 w2, x2 w1; x2 w2, x1 w3, x3 w1): what is left out is about 2^-26 of |x w|, with either sign.
+// are taken (x1 w1; x1 w2, x2 w1; x2 w2, x1 w3, x3 w1): what is left out is 2^-23 of |x w| at most, about 2^-26.7 on average
+// and with either sign.  (x2 w3 and x3 w2 too: 1.10e-7 to 1.09e-7 below, 677 x 1,024 x 6,144 61 to 69 us.)
 // Products of bfloat16 are exact in float32; the tensor cores add them up in tensor memory over 64 k, the small ones
 // first, and every such sum is then added by the float32 cores to a sum in registers, in ascending order of k: the
 // tensor cores cut off what does not fit instead of rounding it, which over all of k would shrink the sums.
 //
 // The sum of an output element has one order whatever m is: blocks of 64 k ascending inside a group of 1,024, the groups
-// ascending.  Infinities, NaN and values from 2^111 on have no such three parts, and a sum of 2^96 and more is beyond float32
-// with the factors (or NaN: x1 w2 may have the other sign than x1 w1).  All of it ends in a sum that is not finite: such an element is summed again by the float32 cores from the operands themselves, and has
-// their bits.
+// ascending.  It is not the order of gemm_simt.cu: an element's last bits depend on which of the two kernels takes the product.
+// Infinities, NaN and values from 2^111 on have no such three parts, and a sum of 2^96 and more is beyond float32 with the
+// factors (or NaN: x1 w2 may have the other sign than x1 w1).  All of it ends in a sum that is not finite: such an element is
+// summed again by the float32 cores from the operands themselves, and has their bits.
+//
+// Error against 64-bit sums (2-norm, 1e-8; this / float32 cores), normal operands at k = 4, 8, 16, 64, 256, 1,024, 3,072, 25,600:
+// 4.9 / 4.1, 4.9 / 4.8, 5.0 / 6.0, 7.9 / 10.7, 8.9 / 15.0, 11.0 / 15.5, 11.6 / 16.0, 14.6 / 20.1; of that 6 is what the tensor
+// cores cut off.  Rows of one value (k = 64, 1,024): 5.2 / 23, 13 / 47.  Where all products have one sign the cuts add up: uniform
+// operands in (0, 1) 8.4 / 6.7, 9.6 / 5.1, 8.9 / 4.9 at k = 64, 1,024, 3,072, and with few products that are most of the sum
+// (e to twice a normal value, both operands) 53 / 10 at k = 64, 37 / 11 at 1,024; with weights of either sign 12 / 14 there.
 //
 // x is split once, by a small kernel; w on its way into shared memory, by the 16 warps that also add up the sums: its
 // parts are never in memory, and a weight takes no more room than before.  Integer instructions split (the conversion
@@ -25,9 +33,8 @@
 // one lane that tells the others: 1.4 and 1.9.)
 //
 // Measured (us, float32 cores / this, weights from memory): 64 rows 4,096 x 1,024 31 / 25, 6,144 x 1,024 43 / 26, 1,024 x
-// 3,072 30 / 27; 301 rows 93 / 30, 127 / 32, 76 / 32; 677 rows 176 / 56, 260 / 63 (136 TFLOP/s), 139 / 40; 2,048 rows
-// 464 / 121, 687 / 176 (147 TFLOP/s), 354 / 104.  Error against 64-bit sums (2-norm) at k = 1,024 / 3,072 / 25,600: 1.10e-7,
-// 1.16e-7, 1.46e-7 (float32 cores 1.55e-7, 1.60e-7, 2.02e-7); of that 6e-8 is what the tensor cores cut off.
+// 3,072 30 / 27; 301 rows 93 / 30, 127 / 32, 76 / 32; 677 rows 176 / 54, 260 / 61 (140 TFLOP/s), 139 / 37; 2,048 rows
+// 464 / 119, 687 / 175 (147 TFLOP/s), 354 / 104.
 #include <algorithm>
 #include <initializer_list>
 

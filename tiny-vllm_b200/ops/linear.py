@@ -1,8 +1,8 @@
 """x . W^T for the parts, by storage dtype.
 
 float32: the package's own kernels, true 32-bit: up to F32_CORE_ROWS rows and narrow products on the float32 cores, the others
-on the tensor cores with every operand as three bfloat16 (each of the two gives a row the same bits whatever else is in the
-batch).
+on the tensor cores with every operand as three bfloat16.  Each of the two gives a row the same bits whatever else is in the
+batch, but not each other's: a row's last bits change between 32 and 33 rows and wherever else the kernel does.
 bfloat16: the tensor-core kernels of this package where they take the shape,
 else cuBLAS through ``torch.nn.functional.linear``, which is what the
 reference's engine calls for every projection (tinyvllm/layers.py:84-85).
