@@ -18,7 +18,6 @@ max(0, p - window + 1) to p through the block table.
 
 from __future__ import annotations
 
-import contextlib
 import math
 import os
 
@@ -176,17 +175,6 @@ def prefill_tiles(counts, starts=None, *, tensor_memory: bool = False, singles_a
     return big, rest, tuple((first, count) for first, count in runs)
 
 
-@contextlib.contextmanager
-def _branch(side):
-    """Launches inside go to the stream ``side`` (None: nowhere else), behind what was launched so far."""
-    if side is None:
-        yield
-        return
-    side.wait_stream(torch.cuda.current_stream(side.device))
-    with torch.cuda.stream(side):
-        yield
-
-
 def mixer_attention(ctx, mixer, qkv: torch.Tensor, run: int) -> torch.Tensor:
     """From the packed projection ``qkv`` [tokens, (q + 2 kv) * head_dim] of a step to the
     attention output [tokens, q * head_dim]; writes the step's keys and values."""
@@ -229,14 +217,8 @@ def mixer_attention(ctx, mixer, qkv: torch.Tensor, run: int) -> torch.Tensor:
     if (tiled and ctx.tile_row is not None
             and kernels.attention_prefill_supports(mixer.head_dim, mixer.num_heads, mixer.num_kv_heads)):
         out = torch.empty((qkv.shape[0], mixer.num_heads * mixer.head_dim), dtype=qkv.dtype, device=qkv.device)
-        # In a recorded step the single tokens are a branch beside the tiles: the decode kernel is bound by memory and by
-        # the steps inside its clusters, the tile kernels by their longest item (24 single tokens beside 798 of prompts:
-        # 31 us and 17 us a layer in line, 42 us this way: the tiles' CTAs find room as the others leave).  Both read
-        # what the preparing kernel stored and write rows of their own.  (Eager steps are bound by their launches.)
-        side = None
-        if ctx.single_runs and ctx.tile_row.shape[0] + (0 if ctx.tile_tc_row is None else ctx.tile_tc_row.shape[0]) > 0:
-            side = ctx.side_stream
-        with _branch(side):
+
+        def single_tokens():
             for first, count in ctx.single_runs:
                 # Decoded tokens beside the portions.  Their q is normalised and rotated and their k, v are
                 # in the cache already, so the fused decode kernel runs without its norm, rotation and
@@ -264,7 +246,19 @@ def mixer_attention(ctx, mixer, qkv: torch.Tensor, run: int) -> torch.Tensor:
                     qkv[part], qkv.shape[1], keys, values, ctx.block_tables[group], ctx.token_row[part],
                     ctx.positions[part], **heads, window=mixer.window, scale=mixer.scale, out=out[part],
                     scratch=scratch, max_chunks=chunks)
-        if ctx.tile_tc_row is not None and ctx.tile_tc_row.shape[0] > 0:
+
+        # In a recorded step the single tokens are a branch beside the tiles: the decode kernel is bound by memory and by
+        # the steps inside its clusters, the tile kernels by their longest item (24 single tokens beside 798 of prompts:
+        # 31 us and 17 us a layer in line, 42 us this way: the tiles' CTAs find room as the others leave).  Both read
+        # what the preparing kernel stored and write rows of their own.  An eager step is bound by its launches and runs
+        # them behind the tiles.
+        tc_tiles = ctx.tile_tc_row is not None and ctx.tile_tc_row.shape[0] > 0
+        side = ctx.side_stream if ctx.single_runs and (tc_tiles or ctx.tile_row.shape[0] > 0) else None
+        if side is not None:
+            side.wait_stream(torch.cuda.current_stream(side.device))
+            with torch.cuda.stream(side):
+                single_tokens()
+        if tc_tiles:
             # the step's tile lists were cut for the tcgen05 kernel: every mixer of the model takes it
             kernels.attention_prefill_tc(
                 qkv, qkv.shape[1], keys, values, ctx.block_tables[group], ctx.positions, ctx.tile_tc_row,
@@ -273,7 +267,9 @@ def mixer_attention(ctx, mixer, qkv: torch.Tensor, run: int) -> torch.Tensor:
             kernels.attention_prefill(
                 qkv, qkv.shape[1], keys, values, ctx.block_tables[group], ctx.positions, ctx.tile_row,
                 ctx.tile_first, ctx.tile_count, **heads, window=mixer.window, scale=mixer.scale, out=out)
-        if side is not None:
+        if side is None:
+            single_tokens()
+        else:
             torch.cuda.current_stream(side.device).wait_stream(side)
         return out
     scratch = None
