@@ -69,3 +69,23 @@ def test_replayed_mixed_steps_equal_eager_ones(model_folders, monkeypatch, name,
                        for kind in ("tiles", "singles")}
             assert len(streams["tiles"]) == len(streams["singles"]) == 1 and streams["tiles"] != streams["singles"]
     assert graphed._step_graphs
+
+
+def test_a_failed_recording_leaves_the_step_on_one_stream(model_folders, monkeypatch):
+    runner = recording(make_runner(model_folders["e"], torch.bfloat16, 16, 64))
+    vocab, forward, seen = TINY_CONFIGS["e"].vocab_size, runner.model.forward, []
+
+    def fails_while_recorded(ctx):
+        if torch.cuda.is_current_stream_capturing():
+            seen.append(ctx)
+            assert ctx.side_stream is not None
+            raise RuntimeError("a part that cannot be recorded")
+        assert ctx.side_stream is None
+        return forward(ctx)
+
+    want = mixed_step(runner, vocab, 0)
+    monkeypatch.setattr(runner.model, "forward", fails_while_recorded)
+    for turn in (0, 0):
+        got = mixed_step(runner, vocab, turn)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert seen and seen[0].side_stream is None and not runner._step_graphs

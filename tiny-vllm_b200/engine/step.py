@@ -442,11 +442,12 @@ class StepRunner:
             except Exception:                             # noqa: BLE001 (reported by the next real call)
                 pass
             return
+        finally:
+            ctx.side_stream = None
         if self._step_graph_pool is None:
             self._step_graph_pool = graph.pool()
         guarded = (after[0] > before[0], after[1] > before[1])      # what one pass of the step launched
         ctx.workspace_of = None       # a replay asks for no scratch; without it the graph does not hold the runner
-        ctx.side_stream = None
         self._step_graphs[ctx.signature] = _StepGraph(graph, ctx.arena, logits, ctx, self._step_count, guarded)
 
     def drop_graphs(self) -> None:
