@@ -2,7 +2,7 @@
 // 32-bit path (no tensor cores, no reduced-precision mode), for any M, N, K.
 //
 // float32 operands.  The sum of an output element has one order, whatever M is and whichever of the
-// two kernels below runs: K is cut into segments of 128; a segment is a chain over its even k and one over
+// two kernels below (float32 cores) runs: K is cut into segments of 128; a segment is a chain over its even k and one over
 // its odd k (one fused multiply-add per k, ascending; the packed instruction on pairs of floats does both),
 // then their sum; four segments are added in ascending order to a group, the groups in ascending
 // order to the result.  A row's result does not depend on which other rows are in the batch, and
@@ -11,7 +11,8 @@
 //
 //  * gemm_f32_few_kernel: up to 8 rows (decode).  Bound by reading W once: x stays in shared memory, W comes
 //    through a ring of cp.async stages of 8 or 16 columns x 1,024 k, a thread owns one (column, segment).
-//  * gemm_f32_tile_kernel: more rows.  Bound by the float32 cores: tiles of up to 64 x 64, a thread
+//  * gemm_f32_tile_kernel: more rows (beyond 32 narrow products and rows off the 16-byte boundary; the others have
+//    gemm_f32_tc.cu, in another order).  Bound by the float32 cores: tiles of up to 64 x 64, a thread
 //    owns up to 8 x 4 outputs, three to four stages of 32 k in flight, groups of 512 k spread over the grid
 //    where the tiles alone leave SMs idle (their sums meet in a second kernel, in the fixed order).
 //
