@@ -29,3 +29,21 @@ def test_route(monkeypatch, sizes, kernel):
     # rows off the 16-byte boundary are the float32 cores' in any case
     linear(torch.empty(m * k + 1)[1:].view(m, k).as_subclass(OnGpu), torch.empty(n, k))
     assert taken[1] == "gemm_nt_simt"
+
+
+@pytest.mark.parametrize("shape,dtype,kernel", [((64, 6144), torch.float32, "gemm_f32_tc"), ((70, 6144), torch.float32, "gemm_nt_simt"),
+                                                ((64, 6150), torch.float32, "gemm_nt_simt"), ((64, 6144), torch.bfloat16, "gemm_nt_simt")])
+def test_a_result_inside_a_larger_tensor_or_of_another_type(monkeypatch, shape, dtype, kernel):
+    """The float32 cores' kernels write the first rows and columns of whatever they are given."""
+    taken = []
+    for name in ("gemm_f32_tc", "gemm_nt_simt"):
+        monkeypatch.setattr(kernels, name, lambda *args, name=name, **words: taken.append(name))
+    linear(torch.empty(64, 1024).as_subclass(OnGpu), torch.empty(6144, 1024), out=torch.empty(shape, dtype=dtype))
+    assert taken == [kernel]
+
+
+def test_operands_that_are_not_matrices_are_refused_as_ever(monkeypatch):
+    monkeypatch.setattr(kernels, "_need_cuda", lambda *tensors: None)
+    for x in (torch.tensor(1.0), torch.empty(1024), torch.empty(2, 40, 1024)):
+        with pytest.raises(kernels.KernelError):
+            linear(x.as_subclass(OnGpu), torch.empty(6144, 1024))

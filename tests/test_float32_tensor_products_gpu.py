@@ -124,9 +124,9 @@ def same_where_not_finite(got, want):
         got == float("-inf"), want == float("-inf"))
 
 
-@pytest.mark.parametrize("m,n,k", [(40, 130, 64), (150, 140, 1028), (150, 140, 2048), (2500, 1500, 2052)])
+@pytest.mark.parametrize("m,n,k", [(40, 130, 64), (150, 140, 1028), (150, 140, 2048), (2500, 1500, 2052), (1100, 40, 25600)])
 def test_products_beyond_float32_are_summed_as_the_float32_cores_do(m, n, k):
-    """Finite operands whose products, or parts' products, leave float32: whole, cut and added up from partial sums."""
+    """Finite operands whose products, or parts' products, leave float32: whole, cut and added up from partial sums, in ranges of rows."""
     generator = torch.Generator(device=DEV).manual_seed(k)
     a, w = torch.randn(m, k, generator=generator, device=DEV), torch.randn(n, k, generator=generator, device=DEV)
     a, w = a + a.sign(), w + w.sign()                       # none near zero: every product below is beyond float32

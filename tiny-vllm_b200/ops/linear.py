@@ -56,7 +56,9 @@ def _tensor_cores_are_quicker(rows: int, columns: int, k: int) -> bool:
 
 
 def _linear_f32(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor | None, weight_constant: bool) -> torch.Tensor:
-    if (x.shape[0] > F32_CORE_ROWS and kernels.gemm_f32_tc_takes(x, weight)
+    # (an ``out`` that is larger than the result, or of another type, is written by the float32 cores' kernels alone)
+    if (x.dim() == 2 and x.shape[0] > F32_CORE_ROWS and kernels.gemm_f32_tc_takes(x, weight)
+            and (out is None or (out.dtype == torch.float32 and out.shape == (x.shape[0], weight.shape[0])))
             and _tensor_cores_are_quicker(x.shape[0], weight.shape[0], x.shape[1])):
         return kernels.gemm_f32_tc(x, weight, out=out, weight_constant=weight_constant)
     return kernels.gemm_nt_simt(x, weight, out=out, weight_constant=weight_constant)
